@@ -65,6 +65,7 @@ int peer_device_status();
 int peer_allreduce_f16(const void *const *bufs, void *const *res, void *const *flags, int rank, int world, void *out, int64_t count,
                        void *state, cudaStream_t st);
 int rtn_device_status();
+int grad_device_status();
 long long div_self_check(unsigned long long n, unsigned long long seed);
 int qmatmul_grad_input(const void *go, int dtype, int64_t M, int64_t N, int64_t K, const int32_t *q,
                        const __half *scale, const __half *zp, void *gi, int bits, int g, cudaStream_t st);
@@ -507,9 +508,10 @@ const char *bw_last_cuda_error(void) { return g_cuda_error; }
 
 int bw_device_status(void) {
     if (cudaDeviceSynchronize() != cudaSuccess) return record_cuda_error(cudaGetLastError(), "cudaDeviceSynchronize");
-    const int v = rtn_device_status(), t = tc_device_status(), d = decode_device_status(), pr = peer_device_status();
-    if (v < 0 || t < 0 || d < 0 || pr < 0) return BW_ERR_CUDA;
-    return (v || t || d || pr) ? BW_ERR_TIMEOUT : BW_OK;
+    const int v = rtn_device_status(), t = tc_device_status(), d = decode_device_status(), pr = peer_device_status(),
+              gr = grad_device_status();
+    if (v < 0 || t < 0 || d < 0 || pr < 0 || gr < 0) return BW_ERR_CUDA;
+    return (v || t || d || pr || gr) ? BW_ERR_TIMEOUT : BW_OK;
 }
 int bw_version(void) { return 100; }
 const char *bw_last_qmatmul_kernel(void) { return g_last_kernel; }

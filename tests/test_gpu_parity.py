@@ -583,6 +583,31 @@ def test_grad_input_tensor_core_kernel_vs_oracle(bits, g, gdt, shape):
     assert bool(((gi.float() - full).abs() <= 1e-2 * rms(as_f32(full)) + slack).all())
 
 
+@pytest.mark.parametrize("bits,g,gdt", [(2, 16, torch.float16), (2, 128, torch.bfloat16), (4, 32, torch.float16), (4, 128, torch.float16),
+                                        (4, 64, torch.bfloat16), (8, 16, torch.bfloat16), (8, 32, torch.float16), (8, 256, torch.float16)])
+def test_grad_input_tiles_match_float64(bits, g, gdt):
+    # token tiles of 16 .. 256 and their remainders, a last column tile and a last stage of rows that are not
+    # whole, rows split over a cluster, several tiles per CTA, scales that TMA can fetch (groups a multiple of 8) or not
+    for M, N, K in ((1, 8, 256), (16, 64, 512), (17, 72, 768), (33, 1000, 512), (64, 4096, 1024), (65, 136, 1280), (129, 520, 2048),
+                    (256, 64, 256 + (128 if g <= 128 else 256)), (257, 1032, 1024), (1030, 256, 8192 + 256)):
+        gen = torch.Generator(device=DEV).manual_seed(M + bits)
+        q = torch.randint(-2 ** 31, 2 ** 31 - 1, (N, K * bits // 32), generator=gen, device=DEV, dtype=torch.int32)
+        s = (torch.rand(N, K // g, generator=gen, device=DEV) * 0.02 + 0.001).half()
+        z = torch.randint(0, 2 ** bits, (N, K // g), generator=gen, device=DEV).half()
+        if M in (17, 129):
+            z[::3] += 0.3125                            # not a whole number: accepted by this entry point
+        go = torch.randn(M, N, generator=gen, device=DEV).to(gdt)
+        w = dequantize_rtn(q, s, z, g, bits=bits).to(gdt).double()
+        ref = go.double() @ w
+        gi = quantized_matmul_grad_input(go, q, s, z, bits, g).double()
+        # one rounding of the result, and fp32 sums that the tensor core truncates once per 16 terms, each
+        # partial sum of the order of |go| . |W|
+        slack = 2.0 ** (-8 if gdt == torch.bfloat16 else -11) * ref.abs() + N / 16 * 2.0 ** -23 * (go.double().abs() @ w.abs()) + 1e-7
+        bad = (gi - ref).abs() > slack
+        assert not bool(bad.any()), (bits, g, M, N, K, int(bad.sum()), float((gi - ref).abs().max()))
+    assert _lib.lib().bw_device_status() == 0
+
+
 @pytest.mark.parametrize("pinned", [True, False])
 @pytest.mark.parametrize("M,N,K,bits,g", [(1, 1024, 4096, 4, 128), (16, 4096, 4096, 4, 128), (5, 72, 256, 8, 32),
                                           (200, 512, 1024, 2, 64)])
