@@ -355,6 +355,194 @@ rtn_quantize_pack_kernel(const T *__restrict__ w, int64_t total_chunks, int cpg_
     }
 }
 
+// ---- wide form: 64 bytes of one group per thread -----------------------------------------------
+//
+// The pass is bound by instruction issue before it is bound by HBM, and most of a 16-byte chunk's
+// instructions do not depend on how many weights the thread holds: the shuffles of the group
+// reduction, the group's parameters (computed by every lane), addresses and stores.  So a thread
+// takes 64 consecutive bytes of one group (32 16-bit or 16 fp32 weights, two 32-byte loads), which
+// also gives it whole packed words: no shuffles assemble them.  A group is g*sizeof(T)/64 lanes.
+//
+// Codes on the fp32 path: the reference's code is rint(RN(RN(v/s) + zp)).  t = RN(v*r + zp) with
+// r = RN(1/s) differs from the value inside rint() by at most 2.5 * 2^(BITS-24) while |v/s| <=
+// 2^BITS (r: 2^BITS * 2^-24; three roundings of half an ulp of 2^BITS), so unless t lies within
+// EPS = 2^(BITS-22) of a tie both round to the same integer -- and that integer needs no clamp when the
+// group's range contains zero (the value then lies in [-1/2, Qmax + 1/2]).  A thread with a weight in
+// that margin (1 in 8000 weights at 8 bits, 1 in 130000 at 4) and warps with a group on one side of
+// zero take the exact quotient (div_by_recip) and the clamps instead.
+__device__ __forceinline__ void load_64(const void *p, uint32_t (&r)[16]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(r[8 * h]), "=r"(r[8 * h + 1]), "=r"(r[8 * h + 2]), "=r"(r[8 * h + 3]),
+                       "=r"(r[8 * h + 4]), "=r"(r[8 * h + 5]), "=r"(r[8 * h + 6]), "=r"(r[8 * h + 7])
+                     : "l"(reinterpret_cast<const unsigned char *>(p) + 32 * h));
+}
+// min / max that keep NaN, as amin / amax do
+__device__ __forceinline__ float min_nan(float a, float b) { float d; asm("min.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b)); return d; }
+__device__ __forceinline__ float max_nan(float a, float b) { float d; asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b)); return d; }
+template <typename T> __device__ __forceinline__ void unit_minmax(const uint32_t (&raw)[16], float &mn, float &mx);
+template <> __device__ __forceinline__ void unit_minmax<float>(const uint32_t (&raw)[16], float &mn, float &mx) {
+    mn = mx = __uint_as_float(raw[0]);
+#pragma unroll
+    for (int i = 1; i < 16; ++i) { mn = min_nan(mn, __uint_as_float(raw[i])); mx = max_nan(mx, __uint_as_float(raw[i])); }
+}
+template <> __device__ __forceinline__ void unit_minmax<__half>(const uint32_t (&raw)[16], float &mn, float &mx) {
+    const __half2 *h = reinterpret_cast<const __half2 *>(raw);
+    __half2 lo = h[0], hi = h[0];
+#pragma unroll
+    for (int i = 1; i < 16; ++i) { lo = __hmin2_nan(lo, h[i]); hi = __hmax2_nan(hi, h[i]); }
+    mn = min_nan(__low2float(lo), __high2float(lo));
+    mx = max_nan(__low2float(hi), __high2float(hi));
+}
+template <> __device__ __forceinline__ void unit_minmax<__nv_bfloat16>(const uint32_t (&raw)[16], float &mn, float &mx) {
+    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(raw);
+    __nv_bfloat162 lo = h[0], hi = h[0];
+#pragma unroll
+    for (int i = 1; i < 16; ++i) { lo = __hmin2_nan(lo, h[i]); hi = __hmax2_nan(hi, h[i]); }
+    mn = min_nan(__low2float(lo), __high2float(lo));
+    mx = max_nan(__low2float(hi), __high2float(hi));
+}
+// weights 2i and 2i+1 of the unit
+template <typename T> __device__ __forceinline__ float2 unit_pair(const uint32_t (&raw)[16], int i);
+template <> __device__ __forceinline__ float2 unit_pair<float>(const uint32_t (&raw)[16], int i) {
+    return make_float2(__uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1]));
+}
+template <> __device__ __forceinline__ float2 unit_pair<__half>(const uint32_t (&raw)[16], int i) {
+    return __half22float2(*reinterpret_cast<const __half2 *>(&raw[i]));
+}
+template <> __device__ __forceinline__ float2 unit_pair<__nv_bfloat16>(const uint32_t (&raw)[16], int i) {
+    return make_float2(__uint_as_float(raw[i] << 16), __uint_as_float(raw[i] & 0xffff0000u));
+}
+template <typename T> struct Unit { static constexpr int E = 64 / sizeof(T); };   // weights per thread
+
+template <typename T, bool NATIVE, int BITS, typename ST, typename ZT>
+__device__ __forceinline__ void rtn_unit(const uint32_t (&raw)[16], int64_t u, bool in_range, int lane, int lpg, int lpg_log2,
+                                         float floor_s, int32_t *__restrict__ qweight, ST *__restrict__ scale,
+                                         ZT *__restrict__ zp) {
+    constexpr int E = Unit<T>::E, VPI = 32 / BITS, NW = E / VPI;
+    constexpr float QMAX = (float)((1 << BITS) - 1);
+    constexpr float MAGIC = 12582912.0f;                 // 1.5 * 2^23
+    constexpr uint32_t MAGIC_BITS = 0x4B400000u;
+    constexpr float EPS = 1.0f / (float)(1 << (22 - BITS));
+    float mn, mx;
+    unit_minmax<T>(raw, mn, mx);
+    for (int off = lpg >> 1; off > 0; off >>= 1) {
+        mn = min_nan(mn, __shfl_xor_sync(0xffffffffu, mn, off));
+        mx = max_nan(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    }
+    // (false for NaN, Inf and weights beyond +-2^40)
+    bool fast = (mn >= -1.0995116e12f) && (mx <= 1.0995116e12f);
+    const bool one_sided = __any_sync(0xffffffffu, fast && !(mn <= 0.0f && mx >= 0.0f));
+    float s = 0.0f, r = 0.0f, zf = 0.0f;
+    int32_t zi = 0;
+    if (fast) {
+        constexpr float RQ = 1.0f / QMAX;
+        s = rnd<T, NATIVE>(__fsub_rn(mx, mn));
+        s = rnd<T, NATIVE>(div_by_recip(s, QMAX, RQ));
+        if (s < floor_s) s = floor_s;
+        fast = (s >= 9.094947e-13f) && (s <= 1.0995116e12f);  // 2^-40 <= scale <= 2^40
+        r = __frcp_rn(s);
+        float z = rnd<T, NATIVE>(div_by_recip(-mn, s, r));
+        z = fminf(fmaxf(rintf(z), 0.0f), QMAX);
+        zi = (int32_t)z;
+        zf = rnd<T, NATIVE>((float)zi);
+    }
+    uint32_t words[NW];
+    bool done = false;
+    if constexpr (!NATIVE) {
+        if (fast && !one_sided) {
+            float far = 0.0f;                            // largest distance to the nearest integer
+            const float2 r2 = make_float2(r, r), z2 = make_float2(zf, zf);
+#pragma unroll
+            for (int wi = 0; wi < NW; ++wi) {
+                uint32_t acc = 0, bias = 0;
+#pragma unroll
+                for (int i = 0; i < VPI; i += 2) {
+                    const float2 t = ffma2(unit_pair<T>(raw, (wi * VPI + i) / 2), r2, z2);
+                    const float2 m = fadd2(t, make_float2(MAGIC, MAGIC));
+                    const float2 n = fadd2(m, make_float2(-MAGIC, -MAGIC));
+                    const float2 d = ffma2(n, make_float2(-1.0f, -1.0f), t);
+                    far = fmaxf(far, fmaxf(fabsf(d.x), fabsf(d.y)));
+                    const uint32_t mul0 = 1u << (i * BITS), mul1 = 1u << ((i + 1) * BITS);
+                    acc += __float_as_uint(m.x) * mul0;
+                    acc += __float_as_uint(m.y) * mul1;
+                    bias += MAGIC_BITS * mul0 + MAGIC_BITS * mul1;
+                }
+                words[wi] = acc - bias;
+            }
+            done = far < 0.5f - EPS;
+        }
+    }
+    if (!done) {
+        if (fast) {
+#pragma unroll
+            for (int wi = 0; wi < NW; ++wi) {
+                uint32_t acc = 0;
+#pragma unroll
+                for (int i = 0; i < VPI; i += 2) {
+                    const float2 v = unit_pair<T>(raw, (wi * VPI + i) / 2);
+                    float2 t = div_by_recip2(v, s, r);
+                    t.x = rnd<T, NATIVE>(t.x); t.y = rnd<T, NATIVE>(t.y);
+                    t = fadd2(t, make_float2(zf, zf));
+                    t.x = rnd<T, NATIVE>(t.x); t.y = rnd<T, NATIVE>(t.y);
+                    t.x = fminf(fmaxf(t.x, 0.0f), QMAX);
+                    t.y = fminf(fmaxf(t.y, 0.0f), QMAX);
+                    t = fadd2(t, make_float2(MAGIC, MAGIC));
+                    acc |= ((__float_as_uint(t.x) - MAGIC_BITS) << (i * BITS)) | ((__float_as_uint(t.y) - MAGIC_BITS) << ((i + 1) * BITS));
+                }
+                words[wi] = acc;
+            }
+        } else {
+            // step by step, with torch's NaN propagation (amin / amax keep NaN, and so do mn / mx)
+            group_params<T, NATIVE>(mn, mx, QMAX, floor_s, s, zi, zf);
+#pragma unroll 1
+            for (int wi = 0; wi < NW; ++wi) {
+                uint32_t acc = 0;
+#pragma unroll 1
+                for (int i = 0; i < VPI; i += 2) {
+                    uint32_t pr[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) pr[j] = raw[j];
+                    float2 v = make_float2(0.0f, 0.0f);
+#pragma unroll
+                    for (int j = 0; j < E / 2; ++j)
+                        if (j == (wi * VPI + i) / 2) v = unit_pair<T>(pr, j);
+                    acc |= code_of<T, NATIVE>(v.x, s, zf, QMAX) << (i * BITS);
+                    acc |= code_of<T, NATIVE>(v.y, s, zf, QMAX) << ((i + 1) * BITS);
+                }
+#pragma unroll
+                for (int j = 0; j < NW; ++j)
+                    if (j == wi) words[j] = acc;
+            }
+        }
+    }
+    if (!in_range) return;
+    if ((lane & (lpg - 1)) == 0) {
+        const int64_t gidx = u >> lpg_log2;
+        scale[gidx] = from_f32<ST>(s);
+        store_zp<ZT>(zp + gidx, zi);
+    }
+    int32_t *dst = qweight + u * NW;
+    if constexpr (NW == 1) *dst = (int32_t)words[0];
+    else if constexpr (NW == 2) *reinterpret_cast<uint2 *>(dst) = make_uint2(words[0], words[1]);
+    else {
+#pragma unroll
+        for (int j = 0; j < NW; j += 4)
+            *reinterpret_cast<uint4 *>(dst + j) = make_uint4(words[j], words[j + 1], words[j + 2], words[j + 3]);
+    }
+}
+
+template <typename T, bool NATIVE, int BITS, typename ST, typename ZT>
+__global__ void __launch_bounds__(256)
+rtn_quantize_pack_wide_kernel(const T *__restrict__ w, int64_t units, int lpg_log2, float floor_s,
+                              int32_t *__restrict__ qweight, ST *__restrict__ scale, ZT *__restrict__ zp) {
+    const int64_t u = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    uint32_t raw[16] = {};
+    if (u < units) load_64(w + u * Unit<T>::E, raw);
+    rtn_unit<T, NATIVE, BITS, ST, ZT>(raw, u, u < units, threadIdx.x & 31, 1 << lpg_log2, lpg_log2, floor_s, qweight, scale, zp);
+}
+
 // ---- several weight matrices in one launch ---------------------------------------------------
 // The per-layer loops of the callers (bitween/quantizer/quantizer.py:72-80,
 // bitween/gradual/base_wrapper.py:300-311) quantize one layer after the other; for the six or
@@ -370,10 +558,7 @@ struct RtnBatchEntry {
     long long first_block;   // first block index of the matrix in the batched grid
 };
 
-template <typename T, bool NATIVE, int BITS, int L, typename ST, typename ZT>
-__global__ void __launch_bounds__(256)
-rtn_quantize_pack_batch_kernel(const RtnBatchEntry *__restrict__ table, int njobs, int cpg_log2, float floor_s) {
-    constexpr int V = Elems16<T>::V;
+__device__ __forceinline__ int rtn_batch_job(const RtnBatchEntry *__restrict__ table, int njobs) {
     __shared__ int job_s;
     if (threadIdx.x == 0) {
         int lo = 0, hi = njobs - 1;                      // last entry with first_block <= blockIdx.x
@@ -384,7 +569,26 @@ rtn_quantize_pack_batch_kernel(const RtnBatchEntry *__restrict__ table, int njob
         job_s = lo;
     }
     __syncthreads();
-    const RtnBatchEntry e = table[job_s];
+    return job_s;
+}
+
+template <typename T, bool NATIVE, int BITS, typename ST, typename ZT>
+__global__ void __launch_bounds__(256)
+rtn_quantize_pack_wide_batch_kernel(const RtnBatchEntry *__restrict__ table, int njobs, int lpg_log2, float floor_s) {
+    const RtnBatchEntry e = table[rtn_batch_job(table, njobs)];
+    const int64_t u = ((int64_t)blockIdx.x - e.first_block) * 256 + threadIdx.x;
+    const int64_t units = e.chunks / 4;                  // four 16-byte chunks per unit
+    uint32_t raw[16] = {};
+    if (u < units) load_64(reinterpret_cast<const T *>(e.w) + u * Unit<T>::E, raw);
+    rtn_unit<T, NATIVE, BITS, ST, ZT>(raw, u, u < units, threadIdx.x & 31, 1 << lpg_log2, lpg_log2, floor_s, e.q,
+                                      reinterpret_cast<ST *>(e.scale), reinterpret_cast<ZT *>(e.zp));
+}
+
+template <typename T, bool NATIVE, int BITS, int L, typename ST, typename ZT>
+__global__ void __launch_bounds__(256)
+rtn_quantize_pack_batch_kernel(const RtnBatchEntry *__restrict__ table, int njobs, int cpg_log2, float floor_s) {
+    constexpr int V = Elems16<T>::V;
+    const RtnBatchEntry e = table[rtn_batch_job(table, njobs)];
     const T *w = reinterpret_cast<const T *>(e.w);
     const int lane = threadIdx.x & 31;
     const int64_t warp = (((int64_t)blockIdx.x - e.first_block) * blockDim.x + threadIdx.x) >> 5;
@@ -563,8 +767,15 @@ rtn_quantize_pack_general_kernel(const T *__restrict__ w, int64_t num_spans, int
 // per call (BW_RTN_TMA_STREAM); the flag of the call in progress on this thread:
 thread_local bool t_rtn_stream = false;
 // A batched call in progress on this thread: the device table, its length and the grid size.
-struct RtnBatchCall { const RtnBatchEntry *table; int njobs; long long blocks; };
-thread_local RtnBatchCall t_rtn_batch = {nullptr, 0, 0};
+struct RtnBatchCall { const RtnBatchEntry *table; int njobs; long long blocks; bool wide; };
+thread_local RtnBatchCall t_rtn_batch = {nullptr, 0, 0, false};
+
+// The wide form: groups of whole 64-byte units, at most a warp of them, weights aligned to its 32-byte loads
+// and packed words to its 16-byte stores.  (Smaller groups share a unit: 16-byte chunks.)
+inline bool rtn_wide_ok(const void *w, const void *q, size_t elem, int g) {
+    const size_t bytes = (size_t)g * elem, lanes = bytes / 64;
+    return bytes % 64 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && aligned_to(w, 32) && aligned_to(q, 16);
+}
 
 int64_t gcd64(int64_t a, int64_t b) { while (b) { int64_t t = a % b; a = b; b = t; } return a; }
 
@@ -584,6 +795,11 @@ int launch_typed(const T *w, int64_t N, int64_t K, int g, int32_t *q, ST *scale,
     if (t_rtn_batch.njobs > 0) {
         // (the caller has checked that every matrix of the batch takes the fast path)
         if (cpg_log2 < 0) return BW_ERR_UNSUPPORTED;
+        if (t_rtn_batch.wide) {
+            rtn_quantize_pack_wide_batch_kernel<T, NATIVE, BITS, ST, ZT><<<(unsigned)t_rtn_batch.blocks, 256, 0, st>>>(
+                t_rtn_batch.table, t_rtn_batch.njobs, cpg_log2 - 2, floor_s);
+            return check_launch("rtn_quantize_pack_wide_batch_kernel");
+        }
         rtn_quantize_pack_batch_kernel<T, NATIVE, BITS, L, ST, ZT><<<(unsigned)t_rtn_batch.blocks, 256, 0, st>>>(
             t_rtn_batch.table, t_rtn_batch.njobs, cpg_log2, floor_s);
         return check_launch("rtn_quantize_pack_batch_kernel");
@@ -601,6 +817,12 @@ int launch_typed(const T *w, int64_t N, int64_t K, int g, int32_t *q, ST *scale,
             const int64_t grid = tiles < 148 * 3 ? tiles : 148 * 3;
             kern<<<(unsigned)grid, RTN_THREADS, smem, st>>>(w, chunks, tiles, cpg_log2, floor_s, q, scale, zp);
             return check_launch("rtn_quantize_pack_stream_kernel");
+        }
+        if (rtn_wide_ok(w, q, sizeof(T), g)) {
+            const int64_t units = chunks / 4;
+            rtn_quantize_pack_wide_kernel<T, NATIVE, BITS, ST, ZT><<<(unsigned)((units + 255) / 256), 256, 0, st>>>(
+                w, units, cpg_log2 - 2, floor_s, q, scale, zp);
+            return check_launch("rtn_quantize_pack_wide_kernel");
         }
         rtn_quantize_pack_kernel<T, NATIVE, BITS, L, ST, ZT><<<(unsigned)blocks, 256, 0, st>>>(
             w, chunks, cpg_log2, floor_s, q, scale, zp);
@@ -733,6 +955,9 @@ int rtn_quantize_pack_batch(const bw_rtn_job *jobs, int njobs, int w_dtype, int 
         }
         return BW_OK;
     }
+    bool wide = true;
+    for (int j = 0; j < njobs && wide; ++j)
+        wide = jobs[j].N * jobs[j].K == 0 || rtn_wide_ok(jobs[j].w, jobs[j].qweight, dtype_size(w_dtype), g);
     static thread_local RtnBatchEntry host_table[4096];
     long long blocks = 0;
     int used = 0, first = -1;
@@ -742,16 +967,16 @@ int rtn_quantize_pack_batch(const bw_rtn_job *jobs, int njobs, int w_dtype, int 
         if (first < 0) first = j;
         host_table[used++] = {jobs[j].w, jobs[j].qweight, jobs[j].scale, jobs[j].zero_point, chunks, blocks};
         const long long warps = (chunks + 32 * lpt - 1) / (32 * lpt);
-        blocks += (warps + 7) / 8;
+        blocks += wide ? (chunks / 4 + 255) / 256 : (warps + 7) / 8;
     }
     if (used == 0) return BW_OK;
     if (blocks > 0x7fffffff) return BW_ERR_SHAPE;
     // (pageable source: the runtime stages the table before the call returns)
     BW_CUDA_TRY(cudaMemcpyAsync(table_dev, host_table, (size_t)used * sizeof(RtnBatchEntry), cudaMemcpyHostToDevice, st));
-    t_rtn_batch = {reinterpret_cast<const RtnBatchEntry *>(table_dev), used, blocks};
+    t_rtn_batch = {reinterpret_cast<const RtnBatchEntry *>(table_dev), used, blocks, wide};
     const int rc = rtn_quantize_pack(jobs[first].w, w_dtype, jobs[first].N, jobs[first].K, bits, g, jobs[first].qweight,
                                      jobs[first].scale, scale_dtype, jobs[first].zero_point, zp_dtype, flags, st);
-    t_rtn_batch = {nullptr, 0, 0};
+    t_rtn_batch = {nullptr, 0, 0, false};
     return rc;
 }
 

@@ -156,6 +156,68 @@ def test_rtn_streaming_kernel_equals_register_kernel(dt):
     assert _bits_equal(got[0][:16], qo) and _bits_equal(got[1][:16], so) and _bits_equal(got[2][:16], zo)
 
 
+def _awkward_weights(N, K, g, bits, dt, seed):
+    """Groups whose quotients lie on and within a few ulps of rounding ties, one-sided ranges, constants,
+    NaN / Inf, and scales near and beyond both ends of the fast path's range."""
+    rng = np.random.default_rng(seed)
+    qmax = 2 ** bits - 1
+    w = np.empty((N * K // g, g), dtype=np.float32)
+    for j in range(w.shape[0]):
+        kind = j % 9
+        s = np.float32(2.0 ** rng.integers(-12, -4)) * np.float32(rng.choice([1.0, 0.7853982, 1.1]))
+        z = int(rng.integers(0, qmax + 1))
+        codes = rng.integers(0, qmax + 1, g).astype(np.float32) - z
+        codes[0], codes[-1] = -z, qmax - z
+        v = codes * s
+        if kind in (0, 1, 2):                     # ties, then ties moved by a few ulps
+            v = (np.clip(codes + 0.5, -z, qmax - z) * s).astype(np.float32)
+            v[0], v[-1] = -z * s, (qmax - z) * s
+            if kind == 1:
+                v = (v.view(np.int32) + rng.integers(-3, 4, g).astype(np.int32) * (v != 0)).view(np.float32)
+            elif kind == 2:
+                v = v * np.float32(1.0 + 2.0 ** -21)
+        elif kind == 3:
+            v = np.abs(v) + s                     # one-sided
+        elif kind == 4:
+            v = -np.abs(v) - s
+        elif kind == 5:
+            v = np.full(g, 0.125, dtype=np.float32)
+        elif kind == 6:
+            v = v.copy()
+            v[int(rng.integers(0, g))] = rng.choice([np.nan, np.inf, -np.inf])
+        elif kind == 7:
+            v = v * np.float32(rng.choice([1e-9, 1e-30, 1e15]))
+        else:
+            v = rng.standard_normal(g).astype(np.float32) * s
+        w[j] = v
+    return torch.from_numpy(w.reshape(N, K)).to(dt)
+
+
+@pytest.mark.parametrize("bits", [2, 4, 8])
+@pytest.mark.parametrize("dt", [torch.float32, torch.float16, torch.bfloat16], ids=str)
+def test_rtn_wide_units_match_oracle_on_awkward_groups(bits, dt):
+    # 64-byte units (one to 32 lanes a group), a last block that is not whole, and the same weights 16 bytes off
+    # a 32-byte boundary (16-byte chunks): one result, the oracle's, bit for bit
+    for N, K, g in ((7, 512, 32), (3, 1024, 64), (65, 1280, 128), (33, 1024, 512), (3, 2048, 1024), (9, 96, 16)):
+        if g * (4 if dt == torch.float32 else 2) // 64 > 32:
+            continue
+        w = _awkward_weights(N, K, g, bits, dt, 17 * bits + g)
+        qo, so, zo = oracle.quantize_rtn(to_np(w), ORACLE_DT[dt], bits, g)
+        pad = 16 // w.element_size()
+        shifted = torch.empty(N * K + pad, dtype=dt, device=DEV)[pad:].view(N, K).copy_(w)
+        assert shifted.data_ptr() % 32 == 16
+        for dev in (w.to(DEV), shifted):
+            q, s, z, _ = quantize_rtn(dev, bits=bits, group_size=g)
+            assert _bits_equal(q, qo) and _bits_equal(z, zo), (N, K, g)
+            ns = torch.isnan(s.cpu())
+            assert torch.equal(ns, torch.isnan(from_bits(so, dt) if dt != torch.float32 else torch.from_numpy(so)))
+            assert bool((to_np(s) == so)[~ns.numpy()].all()), (N, K, g)
+        up = oracle.quantize_rtn(to_np(w.float()), oracle.F32, bits, g)
+        for dev in (w.to(DEV), shifted):
+            q, _, _ = quantize_rtn_to_module_buffers(dev, bits, g)
+            assert _bits_equal(q, up[0]), (N, K, g)
+
+
 def test_rtn_error_bound_full_size_layer():
     # size-independent property at a full Llama-3-8B shape: |w - dequant| <= scale/2 per element
     torch.manual_seed(0)
