@@ -66,6 +66,52 @@ dequantize_kernel(const int32_t *__restrict__ qweight, const ST *__restrict__ sc
     for (int i = 0; i < VPI; ++i) dst[i] = vals[i];
 }
 
+// The same for what nearly every call has -- groups of a power-of-two number of words and an output
+// that vector stores can reach.  Rows are contiguous and hold whole groups, so the group of word wi is
+// wi >> log2(words per group): no divisions (two 64-bit ones a word above).  A thread takes four words
+// a block apart, all loads first: four independent chains in flight, loads and stores of a warp contiguous.
+template <int BITS, typename ST, typename ZT, typename OutT>
+__global__ void __launch_bounds__(256)
+dequantize_words_kernel(const int32_t *__restrict__ qweight, const ST *__restrict__ scale, const ZT *__restrict__ zp,
+                        int64_t total_words, int wpg_log2, OutT *__restrict__ out) {
+    constexpr int VPI = 32 / BITS, U = 4;
+    constexpr uint32_t MASK = (1u << BITS) - 1u;
+    const int64_t w0 = (int64_t)blockIdx.x * (256 * U) + threadIdx.x;
+    uint32_t word[U];
+    float s[U], z[U];
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+        const int64_t wi = w0 + j * 256;
+        word[j] = 0; s[j] = 0.0f; z[j] = 0.0f;
+        if (wi < total_words) {
+            word[j] = (uint32_t)__ldcs(qweight + wi);
+            s[j] = to_f32<ST>(scale[wi >> wpg_log2]);
+            z[j] = to_f32<ZT>(zp[wi >> wpg_log2]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+        const int64_t wi = w0 + j * 256;
+        if (wi >= total_words) return;
+        alignas(16) OutT vals[VPI];
+#pragma unroll
+        for (int i = 0; i < VPI; ++i)
+            vals[i] = from_f32<OutT>(__fmul_rn(s[j], __fsub_rn((float)((word[j] >> (i * BITS)) & MASK), z[j])));
+        constexpr int BYTES = VPI * sizeof(OutT);
+        unsigned char *dst = reinterpret_cast<unsigned char *>(out + wi * VPI);
+        if constexpr (BYTES == 8) __stcs(reinterpret_cast<uint2 *>(dst), *reinterpret_cast<const uint2 *>(vals));
+        else if constexpr (BYTES == 16) __stcs(reinterpret_cast<uint4 *>(dst), *reinterpret_cast<const uint4 *>(vals));
+        else {
+            const uint32_t *r = reinterpret_cast<const uint32_t *>(vals);   // whole 32-byte sectors per store
+#pragma unroll
+            for (int v = 0; v < BYTES / 32; ++v)
+                asm volatile("st.global.cs.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                             ::"l"(dst + 32 * v), "r"(r[8 * v]), "r"(r[8 * v + 1]), "r"(r[8 * v + 2]), "r"(r[8 * v + 3]),
+                               "r"(r[8 * v + 4]), "r"(r[8 * v + 5]), "r"(r[8 * v + 6]), "r"(r[8 * v + 7]) : "memory");
+        }
+    }
+}
+
 template <int BITS, typename ST, typename ZT, typename OutT>
 int launch4(const int32_t *q, const ST *s, const ZT *z, int64_t N, int64_t K, int g, OutT *out,
             cudaStream_t st) {
@@ -73,6 +119,13 @@ int launch4(const int32_t *q, const ST *s, const ZT *z, int64_t N, int64_t K, in
     const int64_t wpr = K / VPI;
     const int64_t total = N * wpr;
     if (total == 0) return BW_OK;
+    const int wpg = g / VPI;
+    if (g % VPI == 0 && (wpg & (wpg - 1)) == 0 && aligned_to(out, 32) && (total + 1023) / 1024 <= 0x7fffffff) {
+        int sh = 0;
+        while ((1 << sh) < wpg) ++sh;
+        dequantize_words_kernel<BITS, ST, ZT, OutT><<<(unsigned)((total + 1023) / 1024), 256, 0, st>>>(q, s, z, total, sh, out);
+        return check_launch("dequantize_words_kernel");
+    }
     const int64_t blocks = (total + 255) / 256;
     if (blocks > 0x7fffffff) return BW_ERR_SHAPE;
     dequantize_kernel<BITS, ST, ZT, OutT><<<(unsigned)blocks, 256, 0, st>>>(

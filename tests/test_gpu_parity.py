@@ -218,6 +218,21 @@ def test_rtn_wide_units_match_oracle_on_awkward_groups(bits, dt):
             assert _bits_equal(q, up[0]), (N, K, g)
 
 
+@pytest.mark.parametrize("bits", [2, 4, 8])
+def test_dequantize_words_kernel_matches_oracle(bits):
+    # power-of-two words per group, sizes around the four-words-a-thread blocks, aligned and misaligned outputs
+    vpi = 32 // bits
+    for N, K, g in ((1, vpi, vpi), (3, 1024, 128), (129, 32 * vpi, 2 * vpi), (1, 4097 * vpi, vpi), (5, 96 * vpi, 3 * vpi)):
+        gen = torch.Generator().manual_seed(N + K)
+        q = torch.randint(-2 ** 31, 2 ** 31 - 1, (N, K // vpi), generator=gen, dtype=torch.int32)
+        s = torch.rand(N, K // g, generator=gen) * 0.02
+        z = torch.randint(0, 2 ** bits, (N, K // g), generator=gen, dtype=torch.int32)
+        ref = oracle.dequantize_rtn(to_np(q), to_np(s), to_np(z), g, bits)
+        for out_dtype in (torch.float32, torch.float16, torch.bfloat16):
+            got = dequantize_rtn(q.to(DEV), s.to(DEV), z.to(DEV), g, bits=bits, out_dtype=out_dtype)
+            assert torch.equal(got.cpu(), torch.from_numpy(ref).to(out_dtype)), (N, K, g, out_dtype)
+
+
 def test_rtn_error_bound_full_size_layer():
     # size-independent property at a full Llama-3-8B shape: |w - dequant| <= scale/2 per element
     torch.manual_seed(0)
