@@ -13,6 +13,7 @@ import torch
 F32, F16, BF16, I32 = 0, 1, 2, 3
 RTN_UPCAST_F32 = 1
 RTN_TMA_STREAM = 2
+ERR_WORKSPACE = 7
 
 _DTYPE_CODE = {torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16, torch.int32: I32}
 
@@ -153,6 +154,11 @@ def stream_ptr(device):
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
 
 
+def raw_stream(device):
+    """The current stream of `device` as an integer handle."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
 def ptr(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None else None
 
@@ -168,7 +174,7 @@ def workspace(device, nbytes):
     as long as the first capture already saw the largest size it needs."""
     if nbytes == 0:
         return None
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    key = (device.index, raw_stream(device))
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
         if buf is not None:
@@ -176,6 +182,11 @@ def workspace(device, nbytes):
         buf = torch.empty(max(nbytes, 1 << 21), dtype=torch.uint8, device=device)
         _workspaces[key] = buf
     return buf
+
+
+def current_workspace(device, raw_stream):
+    """The scratch `workspace` would return on this stream if it is large enough; None before the first call."""
+    return _workspaces.get((device.index, raw_stream))
 
 
 def last_qmatmul_kernel():

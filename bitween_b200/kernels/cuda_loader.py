@@ -17,7 +17,7 @@ def _as_half(t, name):
     _lib.require_cuda(t, name)
     if t.dtype != torch.float16:
         t = t.to(torch.float16)
-    return t.contiguous()
+    return t if t.is_contiguous() else t.contiguous()
 
 
 def quantized_matmul_cuda(x, qweight, scale, zero_point, bias, bits, group_size, out_dtype=None,
@@ -45,18 +45,21 @@ def quantized_matmul_cuda(x, qweight, scale, zero_point, bias, bits, group_size,
     if x.dtype not in _OUT_DTYPES:
         x = x.to(torch.float16)
     K = x.shape[-1]
-    N = qweight.shape[0]
-    vpi = 32 // bits
-    if qweight.shape[1] * vpi != K:
-        raise ValueError(f"x has {K} input features but qweight packs {qweight.shape[1] * vpi}")
+    N, words = qweight.shape[0], qweight.shape[1]
+    if words * (32 // bits) != K:
+        raise ValueError(f"x has {K} input features but qweight packs {words * (32 // bits)}")
     if group_size < 1 or K % group_size != 0:
         raise ValueError("Group size must be at least 1 and divide in_features.")
-    G = K // group_size
-    if tuple(scale.shape) != (N, G) or tuple(zero_point.shape) != (N, G):
-        raise ValueError(f"scale / zero_point must have shape {(N, G)}")
-    x2 = x.reshape(-1, K).contiguous()
+    groups = (N, K // group_size)
+    if scale.shape != groups or zero_point.shape != groups:
+        raise ValueError(f"scale / zero_point must have shape {groups}")
+    flat = x.dim() == 2
+    x2 = x if flat else x.reshape(-1, K)
+    if not x2.is_contiguous():
+        x2 = x2.contiguous()
     M = x2.shape[0]
-    qweight = qweight.contiguous()
+    if not qweight.is_contiguous():
+        qweight = qweight.contiguous()
     scale = _as_half(scale, "scale")
     zero_point = _as_half(zero_point, "zero_point")
     if bias is not None:
@@ -64,14 +67,18 @@ def quantized_matmul_cuda(x, qweight, scale, zero_point, bias, bits, group_size,
         if bias.numel() != N:
             raise ValueError("bias must have out_features elements")
     dev = x2.device
-    for name, t in (("qweight", qweight), ("scale", scale), ("zero_point", zero_point), ("bias", bias)):
-        if t is not None and t.device != dev:
-            raise RuntimeError(f"`{name}` is on {t.device} but x is on {dev}")
-    if activation not in (None, "relu", "silu_mul"):
-        raise ValueError("activation must be None, 'relu' or 'silu_mul'")
-    if activation == "silu_mul" and N % 4 != 0:
-        raise ValueError("'silu_mul' pairs adjacent weight rows (gate, up): out_features must be a multiple of 4")
-    N_out = N // 2 if activation == "silu_mul" else N
+    if qweight.device != dev or scale.device != dev or zero_point.device != dev or (bias is not None and bias.device != dev):
+        for name, t in (("qweight", qweight), ("scale", scale), ("zero_point", zero_point), ("bias", bias)):
+            if t is not None and t.device != dev:
+                raise RuntimeError(f"`{name}` is on {t.device} but x is on {dev}")
+    N_out = N
+    if activation is not None:
+        if activation not in ("relu", "silu_mul"):
+            raise ValueError("activation must be None, 'relu' or 'silu_mul'")
+        if activation == "silu_mul":
+            if N % 4 != 0:
+                raise ValueError("'silu_mul' pairs adjacent weight rows (gate, up): out_features must be a multiple of 4")
+            N_out = N // 2
     if out is None:
         out = torch.empty((M, N_out), dtype=out_dtype, device=dev)
     else:
@@ -86,18 +93,36 @@ def quantized_matmul_cuda(x, qweight, scale, zero_point, bias, bits, group_size,
             residual = residual.contiguous()
         act = {None: _lib.ACT_NONE, "relu": _lib.ACT_RELU, "silu_mul": _lib.ACT_SILU_MUL}[activation]
         ep = _lib.Epilogue(act, None if residual is None else residual.data_ptr())
-    L = _lib.lib()
-    with torch.cuda.device(dev):
-        ws_bytes = L.bw_qmatmul_workspace_bytes_for(M, N, K, bits, group_size, _lib.dtype_code(x2.dtype),
-                                                    16 if x2.data_ptr() % 16 == 0 else 2)
-        ws = _lib.workspace(dev, ws_bytes)
-        args = (_lib.ptr(x2), _lib.dtype_code(x2.dtype), M, N, K, _lib.ptr(qweight),
-                _lib.ptr(scale), _lib.ptr(zero_point), _lib.ptr(bias), _lib.ptr(out),
-                _lib.dtype_code(out_dtype), bits, group_size)
-        tail = (_lib.ptr(ws), 0 if ws is None else ws.numel(), _lib.stream_ptr(dev))
-        rc = L.bw_qmatmul(*args, *tail) if ep is None else L.bw_qmatmul_fused(*args, ep, *tail)
+    x_code = _lib.dtype_code(x2.dtype)
+    args = (x2.data_ptr(), x_code, M, N, K, qweight.data_ptr(), scale.data_ptr(), zero_point.data_ptr(),
+            None if bias is None else bias.data_ptr(), out.data_ptr(), _lib.dtype_code(out_dtype), bits, group_size)
+    if dev.index == torch.cuda.current_device():
+        rc = _launch(dev, args, ep, x_code)
+    else:
+        with torch.cuda.device(dev):
+            rc = _launch(dev, args, ep, x_code)
     _lib.check(rc)
-    return out.reshape(*x.shape[:-1], N_out)
+    return out if flat else out.reshape(*x.shape[:-1], N_out)
+
+
+def _launch(dev, args, ep, x_code):
+    """bw_qmatmul on the current stream with the stream's workspace.  The size a call needs is only asked for
+    when the library reports that the workspace at hand is too small (nothing has been launched then)."""
+    L = _lib.lib()
+    stream = _lib.raw_stream(dev)
+    ws = _lib.current_workspace(dev, stream)
+    while True:
+        tail = (None, 0, stream) if ws is None else (ws.data_ptr(), ws.numel(), stream)
+        rc = L.bw_qmatmul(*args, *tail) if ep is None else L.bw_qmatmul_fused(*args, ep, *tail)
+        if rc != _lib.ERR_WORKSPACE:
+            return rc
+        M, N, K = args[2:5]
+        need = L.bw_qmatmul_workspace_bytes_for(M, N, K, args[11], args[12], x_code, 16 if args[0] % 16 == 0 else 2)
+        if ws is not None and ws.numel() >= need:
+            return rc
+        ws = _lib.workspace(dev, need)
+        if ws is None:
+            return rc
 
 
 def interleave_gate_up(gate, up):

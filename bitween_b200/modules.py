@@ -73,7 +73,11 @@ class QuantizedLinear(nn.Module):
             self.bias = None
 
     def forward(self, x):
-        out_dtype = getattr(self, "out_dtype", None)   # extension: set layer.out_dtype = torch.bfloat16
+        # extension: set layer.out_dtype = torch.bfloat16.  (Looked up in the places an attribute can be in
+        # before asking nn.Module, whose answer to a missing name is an exception.)
+        out_dtype = None
+        if "out_dtype" in self.__dict__ or hasattr(type(self), "out_dtype"):
+            out_dtype = self.out_dtype
         if out_dtype is None:
             return QuantizedLinearFunction.apply(x, self.qweight, self.scale, self.zero_point, self.bias,
                                                  self.bits, self.group_size)
