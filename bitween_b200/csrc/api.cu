@@ -59,6 +59,10 @@ int fake_quant_native(const void *w, int w_dtype, int64_t N, int64_t K, int bits
                       const void *value, void *dq, void *wq, cudaStream_t st);
 int fake_quant_backward(const void *w, int w_dtype, int64_t N, int64_t K, int bits, int g, const float *scale, const float *zp,
                         const void *value, int value_dtype, const float *grad, float *gscale, float *gzp, cudaStream_t st);
+int group_params(const void *w_min, const void *w_max, int dtype, const float *min_scale, const float *max_scale, int64_t n, int bits,
+                 float *scale, float *zp, float *span, cudaStream_t st);
+int group_params_backward(const void *w_min, const void *w_max, int dtype, const float *scale, const float *zp, const float *span,
+                          int64_t n, int bits, const float *gs, const float *gz, float *gmin, float *gmax, cudaStream_t st);
 size_t peer_flag_bytes();
 size_t peer_state_bytes();
 int peer_device_status();
@@ -435,6 +439,37 @@ int bw_fake_quant_backward(const void *w, int w_dtype, int64_t N, int64_t K, int
         return BW_ERR_ALIGN;
     return fake_quant_backward(w, w_dtype, N, K, bits, group_size, scale, zero_point, value, value_dtype, grad_w_dq, grad_scale,
                                grad_zero_point, (cudaStream_t)stream);
+}
+
+int bw_group_params(const void *w_min, const void *w_max, int w_dtype, const float *min_scale, const float *max_scale, int64_t count,
+                    int bits, float *scale, float *zero_point, float *span, void *stream) {
+    if (bits != 2 && bits != 4 && bits != 8) return BW_ERR_BITS;
+    if (count < 0) return BW_ERR_SHAPE;
+    if (!is_float_dtype(w_dtype)) return BW_ERR_DTYPE;
+    if (count == 0) return BW_OK;
+    if (!w_min || !w_max || !min_scale || !max_scale || !scale || !zero_point || !span) return BW_ERR_NULL;
+    const size_t wa = dtype_size(w_dtype);
+    if (!aligned_to(w_min, wa) || !aligned_to(w_max, wa) || !aligned_to(min_scale, 4) || !aligned_to(max_scale, 4) ||
+        !aligned_to(scale, 4) || !aligned_to(zero_point, 4) || !aligned_to(span, 4))
+        return BW_ERR_ALIGN;
+    return group_params(w_min, w_max, w_dtype, min_scale, max_scale, count, bits, scale, zero_point, span, (cudaStream_t)stream);
+}
+
+int bw_group_params_backward(const void *w_min, const void *w_max, int w_dtype, const float *scale, const float *zero_point,
+                             const float *span, int64_t count, int bits, const float *grad_scale, const float *grad_zero_point,
+                             float *grad_min_scale, float *grad_max_scale, void *stream) {
+    if (bits != 2 && bits != 4 && bits != 8) return BW_ERR_BITS;
+    if (count < 0) return BW_ERR_SHAPE;
+    if (!is_float_dtype(w_dtype)) return BW_ERR_DTYPE;
+    if (count == 0) return BW_OK;
+    if (!w_min || !w_max || !scale || !zero_point || !span || !grad_scale || !grad_zero_point || !grad_min_scale || !grad_max_scale)
+        return BW_ERR_NULL;
+    const size_t wa = dtype_size(w_dtype);
+    if (!aligned_to(w_min, wa) || !aligned_to(w_max, wa) || !aligned_to(scale, 4) || !aligned_to(zero_point, 4) || !aligned_to(span, 4) ||
+        !aligned_to(grad_scale, 4) || !aligned_to(grad_zero_point, 4) || !aligned_to(grad_min_scale, 4) || !aligned_to(grad_max_scale, 4))
+        return BW_ERR_ALIGN;
+    return group_params_backward(w_min, w_max, w_dtype, scale, zero_point, span, count, bits, grad_scale, grad_zero_point,
+                                 grad_min_scale, grad_max_scale, (cudaStream_t)stream);
 }
 
 // ---- peer-memory all-reduce (row-parallel layers on one node) ----

@@ -230,6 +230,44 @@ int launch_v(const void *w, int64_t N, int64_t K, int bits, int g, const float *
     return BW_ERR_DTYPE;
 }
 
+// The per-group parameters of a tuned layer (bitween/wrapper.py:127-140) from the group extrema of the frozen
+// weight and the learnable factors, and their backward: a handful of operations per group, one launch each
+// instead of one per operation (7 forward, 13 backward: at 32 groups a row they cost more than the pass over
+// the weights).  One rounding per operation, in torch's order; the quotients are correctly rounded.
+template <typename T>
+__global__ void __launch_bounds__(256)
+group_params_kernel(const T *__restrict__ w_min, const T *__restrict__ w_max, const float *__restrict__ min_scale,
+                    const float *__restrict__ max_scale, int64_t n, float qmax, float *__restrict__ scale, float *__restrict__ zp,
+                    float *__restrict__ span) {
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const float lo = __fmul_rn(to_f32<T>(w_min[i]), min_scale[i]), hi = __fmul_rn(to_f32<T>(w_max[i]), max_scale[i]);
+    const float d = __fsub_rn(hi, lo);
+    float s = __fdiv_rn(d, qmax);
+    if (s < 1e-8f) s = 1e-8f;                            // torch.clamp(min=1e-8): NaN stays NaN
+    span[i] = d;
+    scale[i] = s;
+    zp[i] = __fdiv_rn(-lo, s);
+}
+// (From what the forward left, not from the factors: an optimizer may have stepped in between.)
+template <typename T>
+__global__ void __launch_bounds__(256)
+group_params_backward_kernel(const T *__restrict__ w_min, const T *__restrict__ w_max, const float *__restrict__ scale,
+                             const float *__restrict__ zp, const float *__restrict__ span, int64_t n, float qmax,
+                             const float *__restrict__ gscale, const float *__restrict__ gzp, float *__restrict__ gmin,
+                             float *__restrict__ gmax) {
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const float s = scale[i], gz = gzp[i];
+    // zero_point = -lo / s
+    const float g_lo = -__fdiv_rn(gz, s);
+    const float gs = __fadd_rn(gscale[i], -__fmul_rn(gz, __fdiv_rn(zp[i], s)));
+    // s = clamp(span / qmax), span = hi - lo: the gradient passes where the clamp does nothing
+    const float g_span = __fdiv_rn(span[i], qmax) >= 1e-8f ? __fdiv_rn(gs, qmax) : 0.0f;
+    gmin[i] = __fmul_rn(__fadd_rn(g_lo, -g_span), to_f32<T>(w_min[i]));
+    gmax[i] = __fmul_rn(g_span, to_f32<T>(w_max[i]));
+}
+
 }  // namespace
 
 int fake_quant_native(const void *w, int w_dtype, int64_t N, int64_t K, int bits, int g, const void *scale, const void *zp,
@@ -278,6 +316,36 @@ int fake_quant_backward(const void *w, int w_dtype, int64_t N, int64_t K, int bi
         case BW_BF16: return launch_bwd_v<__nv_bfloat16>(w, N, K, bits, g, scale, zp, value, value_dtype, grad, gscale, gzp, st);
         default: return BW_ERR_DTYPE;
     }
+}
+
+int group_params(const void *w_min, const void *w_max, int dtype, const float *min_scale, const float *max_scale, int64_t n, int bits,
+                 float *scale, float *zp, float *span, cudaStream_t st) {
+    if (n == 0) return BW_OK;
+    if ((n + 255) / 256 > 0x7fffffff) return BW_ERR_SHAPE;
+    const unsigned blocks = (unsigned)((n + 255) / 256);
+    const float qmax = (float)((1 << bits) - 1);
+    switch (dtype) {
+        case BW_F32: group_params_kernel<float><<<blocks, 256, 0, st>>>((const float *)w_min, (const float *)w_max, min_scale, max_scale, n, qmax, scale, zp, span); break;
+        case BW_F16: group_params_kernel<__half><<<blocks, 256, 0, st>>>((const __half *)w_min, (const __half *)w_max, min_scale, max_scale, n, qmax, scale, zp, span); break;
+        case BW_BF16: group_params_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16 *)w_min, (const __nv_bfloat16 *)w_max, min_scale, max_scale, n, qmax, scale, zp, span); break;
+        default: return BW_ERR_DTYPE;
+    }
+    return check_launch("group_params_kernel");
+}
+
+int group_params_backward(const void *w_min, const void *w_max, int dtype, const float *scale, const float *zp, const float *span,
+                          int64_t n, int bits, const float *gs, const float *gz, float *gmin, float *gmax, cudaStream_t st) {
+    if (n == 0) return BW_OK;
+    if ((n + 255) / 256 > 0x7fffffff) return BW_ERR_SHAPE;
+    const unsigned blocks = (unsigned)((n + 255) / 256);
+    const float qmax = (float)((1 << bits) - 1);
+    switch (dtype) {
+        case BW_F32: group_params_backward_kernel<float><<<blocks, 256, 0, st>>>((const float *)w_min, (const float *)w_max, scale, zp, span, n, qmax, gs, gz, gmin, gmax); break;
+        case BW_F16: group_params_backward_kernel<__half><<<blocks, 256, 0, st>>>((const __half *)w_min, (const __half *)w_max, scale, zp, span, n, qmax, gs, gz, gmin, gmax); break;
+        case BW_BF16: group_params_backward_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16 *)w_min, (const __nv_bfloat16 *)w_max, scale, zp, span, n, qmax, gs, gz, gmin, gmax); break;
+        default: return BW_ERR_DTYPE;
+    }
+    return check_launch("group_params_backward_kernel");
 }
 
 }  // namespace bw

@@ -81,6 +81,10 @@ def _declare(L):
     L.bw_fake_quant_native16.restype = i32
     L.bw_fake_quant_backward.argtypes = [vp, i32, i64, i64, i32, i32, vp, vp, vp, i32, vp, vp, vp, vp]
     L.bw_fake_quant_backward.restype = i32
+    L.bw_group_params.argtypes = [vp, vp, i32, vp, vp, i64, i32, vp, vp, vp, vp]
+    L.bw_group_params.restype = i32
+    L.bw_group_params_backward.argtypes = [vp, vp, i32, vp, vp, vp, i64, i32, vp, vp, vp, vp, vp]
+    L.bw_group_params_backward.restype = i32
     L.bw_dequantize.argtypes = [vp, vp, i32, vp, i32, i64, i64, i32, i32, vp, i32, vp]
     L.bw_dequantize.restype = i32
     L.bw_qmatmul_workspace_bytes.argtypes = [i64, i64, i64, i32, i32]

@@ -111,6 +111,39 @@ def fake_quantize(weight, scale, zero_point, value, bits, group_size, want_q=Tru
     return _FakeQuant.apply(weight.contiguous(), scale, zero_point, value, bits, group_size, want_q)
 
 
+class _GroupParams(torch.autograd.Function):
+    """`WrapperLinear._group_params` with both factors, as one kernel forward and one backward."""
+
+    @staticmethod
+    def forward(ctx, w_min, w_max, min_scale, max_scale, bits):
+        scale = torch.empty_like(min_scale)
+        zero_point = torch.empty_like(min_scale)
+        span = torch.empty_like(min_scale)
+        with torch.cuda.device(w_min.device):
+            rc = _lib.lib().bw_group_params(_lib.ptr(w_min), _lib.ptr(w_max), _lib.dtype_code(w_min.dtype), _lib.ptr(min_scale),
+                                            _lib.ptr(max_scale), w_min.numel(), bits, _lib.ptr(scale), _lib.ptr(zero_point),
+                                            _lib.ptr(span), _lib.stream_ptr(w_min.device))
+        _lib.check(rc)
+        # (not the factors: like the separate ops, this lets an optimizer step before the backward)
+        ctx.save_for_backward(w_min, w_max, scale, zero_point, span)
+        ctx.bits = bits
+        return scale, zero_point
+
+    @staticmethod
+    def backward(ctx, grad_scale, grad_zero_point):
+        w_min, w_max, scale, zero_point, span = ctx.saved_tensors
+        gs, gz = grad_scale.contiguous(), grad_zero_point.contiguous()
+        g_min = torch.empty_like(scale)
+        g_max = torch.empty_like(scale)
+        with torch.cuda.device(w_min.device):
+            rc = _lib.lib().bw_group_params_backward(_lib.ptr(w_min), _lib.ptr(w_max), _lib.dtype_code(w_min.dtype),
+                                                     _lib.ptr(scale), _lib.ptr(zero_point), _lib.ptr(span), w_min.numel(), ctx.bits,
+                                                     _lib.ptr(gs), _lib.ptr(gz), _lib.ptr(g_min), _lib.ptr(g_max),
+                                                     _lib.stream_ptr(w_min.device))
+        _lib.check(rc)
+        return None, None, g_min, g_max, None
+
+
 class WrapperLinear(nn.Module):
     """Drop-in for bitween/wrapper.py:28-242."""
 
@@ -203,8 +236,22 @@ class WrapperLinear(nn.Module):
         # min/max factors in this mode)
         return dq, wq.view(N, K // self.group_size, self.group_size), scale, zero_point
 
+    def _fused_group_params(self):
+        """`_group_params` by one kernel where its operands are what the constructor made them; None otherwise
+        (no factors, a module cast to another dtype, a subclass with parameters of its own)."""
+        lo, hi, a, b = self._w_min, self._w_max, self.min_scale, self.max_scale
+        if a is None or b is None or type(self)._group_params is not WrapperLinear._group_params:
+            return None
+        for t in (lo, hi, a, b):
+            if type(t) not in (torch.Tensor, nn.Parameter) or not t.is_cuda or not t.is_contiguous() or t.shape != lo.shape or t.device != lo.device:
+                return None
+        if a.dtype != torch.float32 or b.dtype != torch.float32 or lo.dtype != hi.dtype or \
+                lo.dtype not in (torch.float32, torch.float16, torch.bfloat16) or lo.requires_grad or hi.requires_grad:
+            return None
+        return _GroupParams.apply(lo, hi, a, b, self.bits)
+
     def forward(self, x):
-        scale, zero_point = self._group_params()
+        scale, zero_point = self._fused_group_params() or self._group_params()
         if scale.dtype != torch.float32:
             weight_dq = self._all_16bit_path(scale, zero_point)[0]
         else:

@@ -310,6 +310,24 @@ BW_API int bw_fake_quant_backward(const void *w, int w_dtype, int64_t N, int64_t
                            float *grad_scale, float *grad_zero_point, void *stream);
 
 /*
+ * The per-group scale and float zero point of a tuned layer (bitween/wrapper.py:127-140),
+ *     lo = w_min * min_scale, hi = w_max * max_scale,
+ *     scale = max((hi - lo) / (2^bits - 1), 1e-8),  zero_point = -lo / scale,
+ * in fp32 with one rounding per operation; span = hi - lo is what the backward needs besides them.
+ * Backward: the gradients of the two factors from those of scale and zero_point (none through the
+ * scale where the floor of 1e-8 holds it).
+ *   w_min, w_max [count] of w_dtype      everything else [count] fp32
+ */
+BW_API int bw_group_params(const void *w_min, const void *w_max, int w_dtype, const float *min_scale,
+                    const float *max_scale, int64_t count, int bits, float *scale, float *zero_point,
+                    float *span, void *stream);
+BW_API int bw_group_params_backward(const void *w_min, const void *w_max, int w_dtype,
+                             const float *scale, const float *zero_point, const float *span,
+                             int64_t count, int bits, const float *grad_scale,
+                             const float *grad_zero_point, float *grad_min_scale,
+                             float *grad_max_scale, void *stream);
+
+/*
  * All-reduce (sum) of the row-parallel layers' partial outputs over peer memory on one node,
  * without NCCL.  No counterpart in the reference (it is single-GPU); it replaces the
  * ncclAllReduce that follows o_proj / down_proj in the tensor-parallel layers of this library.

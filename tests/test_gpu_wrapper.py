@@ -226,3 +226,38 @@ def test_wrap_train_unwrap_block():
     assert isinstance(model["blk"].fc1, QuantizedLinear)
     restored = unified_unwrapper(info["head"]["wrapped_module"], apply_quantization=False)
     assert restored is info["head"]["original_module"]
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.float16, torch.bfloat16], ids=str)
+@pytest.mark.parametrize("bits,N,G", [(2, 1, 1), (4, 255, 3), (8, 513, 16)])
+def test_group_parameter_kernels_equal_the_separate_operations(dt, bits, N, G):
+    # scale and zero point bit for bit; the factors' gradients to a few roundings of their largest term (torch
+    # adds the two contributions to lo in another order); ranges at the 1e-8 floor; an optimizer step in between
+    g = 16
+    gen = torch.Generator(device=DEV).manual_seed(bits)
+    layer = torch.nn.Linear(G * g, N, bias=False, device=DEV, dtype=dt)
+    with torch.no_grad():
+        layer.weight.copy_(torch.randn(N, G * g, generator=gen, device=DEV) * 0.02)
+        if N > 8:
+            layer.weight[3, :g] = 0.0                  # the floor holds the scale
+            layer.weight[5, :g] = 0.25
+    wl = WrapperLinear(layer, bits=bits, group_size=g)
+    with torch.no_grad():
+        wl.min_scale.copy_(torch.rand(N, G, generator=gen, device=DEV) * 0.2 + 0.9)
+        wl.max_scale.copy_(torch.rand(N, G, generator=gen, device=DEV) * 0.2 + 0.9)
+    scale, zp = wl._fused_group_params()
+    scale_t, zp_t = wl._group_params()
+    assert torch.equal(scale, scale_t) and torch.equal(zp, zp_t)
+    gs = torch.randn(N, G, generator=gen, device=DEV)
+    gz = torch.randn(N, G, generator=gen, device=DEV)
+    want = torch.autograd.grad((scale_t, zp_t), (wl.min_scale, wl.max_scale), (gs, gz))
+    with torch.no_grad():
+        wl.min_scale.mul_(1.01)
+    got = torch.autograd.grad((scale, zp), (wl.min_scale, wl.max_scale), (gs, gz))
+    terms = (gs.abs() + gz.abs() * zp.abs() / scale) / (2 ** bits - 1) + gz.abs() / scale
+    for a, b, w in zip(got, want, (wl._w_min, wl._w_max)):
+        assert bool(((a - b).abs() <= 8 * 2.0 ** -24 * terms.detach() * w.float().abs()).all())
+    # not taken: no factors, another dtype, a subclass with its own parameters
+    assert WrapperLinear(layer, bits=bits, group_size=g, enable_minmax_tuning=False)._fused_group_params() is None
+    assert WrapperLinear(layer, bits=bits, group_size=g).half()._fused_group_params() is None
+    assert type("Own", (WrapperLinear,), {"_group_params": lambda self: None})(layer, bits=bits, group_size=g)._fused_group_params() is None
