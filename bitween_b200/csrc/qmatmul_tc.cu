@@ -85,7 +85,7 @@ struct TcParams {
     int persistent;     // 1: grid.x CTAs walk the tile list (tile = blockIdx.x, += gridDim.x); 0: one tile per CTA
     int tma_store;      // 1: output blocks leave through a shared-memory staging tile and TMA stores
     int pdl;            // 1: launched with programmatic stream serialisation behind the kernel that casts the activations
-    int x_is_bf16;      // always 0: kind::f16 MMAs take both operands in one 16-bit format
+    int const_vec;      // 1: rows of scales / zero points are whole 16-byte vectors
     Epilogue ep;        // activation / residual add on the way out
 };
 
@@ -97,21 +97,34 @@ template <int BITS> struct StageGeom {
     static constexpr int SPS = 32 / WPS;              // k-stages per 128-byte row segment of a packed-word slot: 8 / 4 / 2
 };
 
+// Scale (low half) and zero point (high half) of one group.
+__device__ __forceinline__ GroupConst group_const(uint32_t sz) {
+    GroupConst c;
+    c.s2 = __byte_perm(sz, 0, 0x1010);
+    c.z1024 = h2_as_u32(__hadd2(u32_as_h2(__byte_perm(sz, 0, 0x3232)), __float2half2_rn(1024.0f)));
+    return c;
+}
+// Halfword i (0..7) of a 16-byte vector; i is uniform over the warp.
+__device__ __forceinline__ uint32_t half_of(const uint4 &v, int i) {
+    const uint32_t w = (i & 4) ? ((i & 2) ? v.w : v.z) : ((i & 2) ? v.y : v.x);
+    return (i & 1) ? w >> 16 : w & 0xffffu;
+}
+
 // Expands the WPS words of one stage into the row's eight 16-byte chunks (8 consecutive k each).
-// ONE: the whole stage lies in one quantization group (group_size >= 64): no per-word lookup.
+// sz: the stage's groups; ONE: the whole stage lies in one of them (group_size >= 64): no per-word lookup.
 template <int BITS, bool ONE>
-__device__ __forceinline__ void expand_stage(const uint32_t (&w)[StageGeom<BITS>::WPS], const GroupConst (&gc)[4],
-                                             int kbase, int g_shift, int grp0, uint4 (&chunk)[8]) {
+__device__ __forceinline__ void expand_stage(const uint32_t (&w)[StageGeom<BITS>::WPS], const uint32_t (&sz)[4],
+                                             int g_shift, uint4 (&chunk)[8]) {
     constexpr int VPI = 32 / BITS;
     constexpr int WPS = StageGeom<BITS>::WPS;
     Dequant<BITS> dq;
     int cur = -1;
-    if constexpr (ONE) dq.set(gc[0]);
+    if constexpr (ONE) dq.set(group_const(sz[0]));
 #pragma unroll
     for (int j = 0; j < WPS; ++j) {
         if constexpr (!ONE) {
-            const int gl = min(((kbase + j * VPI) >> g_shift) - grp0, 3);
-            if (gl != cur) { dq.set(gc[gl]); cur = gl; }
+            const int gl = (j * VPI) >> g_shift;
+            if (gl != cur) { dq.set(group_const(gl == 0 ? sz[0] : gl == 1 ? sz[1] : gl == 2 ? sz[2] : sz[3])); cur = gl; }
         }
         if constexpr (BITS == 4) {
             uint32_t p[4];
@@ -289,28 +302,52 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
             if (!n_ok) n = p.N - 1;
             const __half *srow = p.scale + n * p.G, *zrow = p.zp + n * p.G;
 
-            GroupConst gcs[4];
-            auto prefetch_consts = [&](int kt) {             // kt = global k-stage index
+            // The row's scales and zero points.  Where rows of them allow 16-byte loads, eight groups at a time,
+            // fetched one stage ahead: at group size 128 a block lasts this group of threads four of its stages.  (Two
+            // 2-byte loads a stage, 32 rows = 32 cache lines each, kept the load/store unit busy for half of a
+            // stage's 512 cycles.)
+            uint4 s_blk = {}, z_blk = {};                    // (s_blk: the next stage's packed pairs when vectors cannot be used)
+            int blk = -1;
+            auto fetch_consts = [&](int kt) {                // kt = global k-stage index
                 const int grp0 = (kt * TC_BK) >> p.g_shift;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    if (i < gps) {
-                        const int grp = min(grp0 + i, p.G - 1);
-                        gcs[i].s2 = h2_as_u32(__half2half2(__ldg(srow + grp)));
-                        gcs[i].z1024 = h2_as_u32(__hadd2(__half2half2(__ldg(zrow + grp)), __float2half2_rn(1024.0f)));
-                    } else {
-                        gcs[i] = gcs[0];
+                if (p.const_vec) {
+                    if ((grp0 >> 3) != blk) {
+                        blk = grp0 >> 3;
+                        s_blk = __ldg(reinterpret_cast<const uint4 *>(srow) + blk);
+                        z_blk = __ldg(reinterpret_cast<const uint4 *>(zrow) + blk);
                     }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (i < gps) {
+                            const int grp = min(grp0 + i, p.G - 1);
+                            (&s_blk.x)[i] = (uint32_t)__ldg(reinterpret_cast<const unsigned short *>(srow) + grp) |
+                                            (uint32_t)__ldg(reinterpret_cast<const unsigned short *>(zrow) + grp) << 16;
+                        }
+                }
+            };
+            // the constants of stage kt, which fetch_consts has been called for
+            auto take_consts = [&](int kt, uint32_t (&sz)[4]) {
+                if (p.const_vec) {
+                    const int grp0 = (kt * TC_BK) >> p.g_shift;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (i < gps) sz[i] = half_of(s_blk, (grp0 + i) & 7) | half_of(z_blk, (grp0 + i) & 7) << 16;
+                        else sz[i] = 0;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) sz[i] = (&s_blk.x)[i];
                 }
             };
             const int i0 = (dgroup - gbase) & (TC_DQ_GROUPS - 1);   // this group's first stage of the tile
-            if (i0 < nk) prefetch_consts(kt0 + i0);
+            if (i0 < nk) fetch_consts(kt0 + i0);
             for (int i = i0; i < nk; i += TC_DQ_GROUPS) {
                 const int gi = gbase + i;
                 const int sa = gi % TC_STAGES;
                 const int kt = kt0 + i;
-                GroupConst gc_now[4] = {gcs[0], gcs[1], gcs[2], gcs[3]};
-                if (i + TC_DQ_GROUPS < nk) prefetch_consts(kt + TC_DQ_GROUPS);
+                uint32_t sz[4];
+                take_consts(kt, sz);
+                if (i + TC_DQ_GROUPS < nk) fetch_consts(kt + TC_DQ_GROUPS);
                 uint32_t w[SG::WPS];
                 {
                     // stage i lies in slot i / SPS of this tile, at position (i % SPS) of each 128-byte row
@@ -332,8 +369,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
                     if (lane == 0) mbar_arrive(&w_empty[si]);    // the packed words are in registers now
                 }
                 uint4 chunk[8];
-                if (gps == 1) expand_stage<BITS, true>(w, gc_now, kt * TC_BK, p.g_shift, (kt * TC_BK) >> p.g_shift, chunk);
-                else expand_stage<BITS, false>(w, gc_now, kt * TC_BK, p.g_shift, (kt * TC_BK) >> p.g_shift, chunk);
+                if (gps == 1) expand_stage<BITS, true>(w, sz, p.g_shift, chunk);
+                else expand_stage<BITS, false>(w, sz, p.g_shift, chunk);
                 ok = __all_sync(0xffffffffu, mbar_wait(&a_empty[sa], ((unsigned)(gi / TC_STAGES) & 1u) ^ 1u, abort_flag, 4));
                 if (!ok) break;
                 tc_fence_after();                            // the MMAs that read this stage come before the stores below
@@ -496,13 +533,21 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
 
 // Activations that are not fp16 are cast once (bitween/modules.py:74) into caller scratch.
 template <typename XT>
-__global__ void __launch_bounds__(256) cast_to_f16_kernel(const XT *__restrict__ x, __half *__restrict__ y, int64_t n) {
+__global__ void __launch_bounds__(256) cast_to_f16_kernel(const XT *__restrict__ x, __half *__restrict__ y, int64_t n, bool vec) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");     // the GEMM behind it may start its set-up
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
     if (i + 8 <= n) {
         alignas(16) __half h[8];
+        alignas(16) XT v[8];
+        if (vec) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) h[j] = from_f32<__half>(to_f32<XT>(x[i + j]));
+            for (int j = 0; j < (int)sizeof(XT) / 2; ++j) reinterpret_cast<uint4 *>(v)[j] = reinterpret_cast<const uint4 *>(x + i)[j];
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = x[i + j];
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) h[j] = from_f32<__half>(to_f32<XT>(v[j]));
         *reinterpret_cast<uint4 *>(y + i) = *reinterpret_cast<const uint4 *>(h);
     } else {
         for (int64_t j = i; j < n; ++j) y[j] = from_f32<__half>(to_f32<XT>(x[j]));
@@ -660,9 +705,9 @@ int qmatmul_tc(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, cons
         const int64_t n = M * K;
         const unsigned blocks = (unsigned)((n / 8 + 255) / 256 + 1);
         switch (x_dtype) {
-            case BW_F16: cast_to_f16_kernel<__half><<<blocks, 256, 0, st>>>((const __half *)x, y, n); break;
-            case BW_BF16: cast_to_f16_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16 *)x, y, n); break;
-            default: cast_to_f16_kernel<float><<<blocks, 256, 0, st>>>((const float *)x, y, n); break;
+            case BW_F16: cast_to_f16_kernel<__half><<<blocks, 256, 0, st>>>((const __half *)x, y, n, false); break;
+            case BW_BF16: cast_to_f16_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16 *)x, y, n, aligned_to(x, 16)); break;
+            default: cast_to_f16_kernel<float><<<blocks, 256, 0, st>>>((const float *)x, y, n, aligned_to(x, 16)); break;
         }
         int rc = check_launch("cast_to_f16_kernel");
         if (rc != BW_OK) return rc;
@@ -678,7 +723,7 @@ int qmatmul_tc(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, cons
     p.words_per_row = (int)(K / (32 / bits));
     p.k_stages = (int)((K + TC_BK - 1) / TC_BK);
     p.bn = M > 128 ? 256 : (M > 64 ? 128 : (M > 32 ? 64 : (M > 16 ? 32 : 16)));
-    p.x_is_bf16 = 0;
+    p.const_vec = p.G % 8 == 0 && aligned_to(scale, 16) && aligned_to(zp, 16) ? 1 : 0;
     p.pdl = direct ? 0 : 1;      // the cast kernel precedes this launch in the stream
     p.ep = current_epilogue();
 
@@ -687,7 +732,7 @@ int qmatmul_tc(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, cons
     const cuuint64_t strides[1] = {(cuuint64_t)K * 2};                 // bytes between token rows
     const cuuint32_t box[2] = {(cuuint32_t)TC_BK, (cuuint32_t)p.bn};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode_tiled_fn()(&map, p.x_is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(xh), dims,
+    const CUresult r = encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(xh), dims,
                                          strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
