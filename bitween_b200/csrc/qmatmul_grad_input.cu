@@ -247,7 +247,7 @@ inline bool grad_tc_ok(const void *go, const void *gi, int dt, int64_t N, int64_
 // bandwidth, not the tensor pipe, sets the pace of 256-token tiles.  Measured: forward and backward of a
 // Llama-3-8B block's seven linears at 2048 tokens (W4 g128, 1.8 TFLOP, half of it here) 11.6 ms with the
 // mma.sync kernel above (which re-expands the weights for every 128 tokens and multiplies at 80 TFLOP/s),
-// 1.88 ms with this one.
+// 1.76 ms with this one.
 constexpr int GU_BK = 128;          // k columns per tile (MMA M)
 constexpr int GU_BN = 64;           // weight rows per stage (reduction)
 constexpr int GU_AS = 4;            // stages of expanded weights == dequantization groups
@@ -388,7 +388,10 @@ grad_input_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_c
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // (Broadcast, so that the compiler knows the roles' branches, loops and addresses to be warp-uniform: the
+    // operands of tcgen05 and mbarrier instructions then stay in uniform registers: 908 -> 740 us for the
+    // seven linears of a Llama-3-8B block at 2048 tokens.)
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int st0 = blockIdx.z * p.per_split;
     const int nk = max(min(st0 + p.per_split, p.steps) - st0, 0);            // stages of this CTA per tile
     const int first_tile = (int)blockIdx.x, tile_step = (int)gridDim.x;
@@ -407,7 +410,7 @@ grad_input_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_c
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
     if (warp == 0) {
         // ---- TMA producer of grad_out tiles [bn tokens x 64 n] ----

@@ -169,7 +169,10 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // (Broadcast, so that the compiler knows the roles' branches, loops and addresses to be warp-uniform: the
+    // operands of tcgen05 and mbarrier instructions then stay in uniform registers and nothing spills.
+    // 14336 x 4096, W4 g128: 819 -> 700 us at 8192 tokens, 62 -> 53 at 509, 25.2 -> 23.9 at 48.)
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     // Tile schedule.  Persistent launches (no split-K) walk the list tile = mt * n_tiles + nt from
     // blockIdx.x in steps of gridDim.x: barriers, rings and tensor memory are set up once, the
     // producer runs ahead into the next tile while the current one drains, and only the epilogue
@@ -201,7 +204,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
     if (warp == 0) {
         // ---- TMA producer of the activation tiles (one thread) ----
@@ -304,8 +307,8 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
 
             // The row's scales and zero points.  Where rows of them allow 16-byte loads, eight groups at a time,
             // fetched one stage ahead: at group size 128 a block lasts this group of threads four of its stages.  (Two
-            // 2-byte loads a stage, 32 rows = 32 cache lines each, kept the load/store unit busy for half of a
-            // stage's 512 cycles.)
+            // 2-byte loads a stage are 32 rows = 32 cache lines each.  8192 tokens through the linears of a
+            // Llama-3-8B block: 3.63 ms with them, 3.55 with these; 48 tokens 484 and 478 us for four blocks.)
             uint4 s_blk = {}, z_blk = {};                    // (s_blk: the next stage's packed pairs when vectors cannot be used)
             int blk = -1;
             auto fetch_consts = [&](int kt) {                // kt = global k-stage index
