@@ -73,6 +73,7 @@ struct DecParams {
     unsigned *cnt;        // this call's slice of g_dec_cnt
     float *part;          // partial tiles [2 * cta + which][MTOK][128] fp32
     const __half *bias;
+    const __half *scale, *zp;   // read directly when they do not come by TMA
     void *out;
     int64_t M, N, K;
     int x_dtype, out_dtype;
@@ -242,7 +243,9 @@ __device__ __forceinline__ int dec_cta_of(int64_t tile, int64_t tiles, int64_t c
 
 // EPI: the output stage applies an activation / residual add (bw_qmatmul_fused); a separate
 // instantiation, so that the plain kernel's code is not touched by it.
-template <int BITS, int MT, bool EPI>
+// CTMA: scales and zero points arrive by TMA with the tile; otherwise (rows of them that are not whole 16-byte
+// units, as for a feed-forward width of 86 groups) each consumer lane loads its own, one tile ahead.
+template <int BITS, int MT, bool EPI, bool CTMA>
 __global__ void __launch_bounds__(DecWarps<MT>::THREADS, 1)
 qmm_decode_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap s_map,
                   const __grid_constant__ CUtensorMap z_map, const __grid_constant__ CUtensorMap x_map,
@@ -260,7 +263,7 @@ qmm_decode_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
     unsigned char *base = smem_dyn + ((1024u - (smem_addr(smem_dyn) & 1023u)) & 1023u);   // swizzled tiles: 1024-byte aligned
     unsigned char *wst = base;                                       // [S][16 KB] packed words
     unsigned char *cst = wst + (size_t)S * DK_W_BYTES;               // [S][scale box 2 KB | zero-point box 2 KB]
-    unsigned char *xst = cst + (size_t)S * 2 * DK_C_BYTES;           // [S][XB] activations in fragment order
+    unsigned char *xst = cst + (size_t)S * (CTMA ? 2 * DK_C_BYTES : 0);   // [S][XB] activations in fragment order
     unsigned char *rst = xst + (size_t)S * XB;                       // [S][raw_bytes] raw activations
     float *red = reinterpret_cast<float *>(rst + (size_t)S * p.raw_bytes);   // [NRED buffers][2 parities][MTOK][128]
     uint64_t *full = reinterpret_cast<uint64_t *>(red + NRED * 2 * RED);
@@ -274,7 +277,7 @@ qmm_decode_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
     float4 *cpart = reinterpret_cast<float4 *>(                      // [cluster ranks][slice] the peers' shares of this CTA's slice of the outputs
         (reinterpret_cast<uintptr_t>(slots + DK_MAX_CTAS) + 15) & ~(uintptr_t)15);
     volatile int *dead = flags;
-    const unsigned stage_tx = DK_W_BYTES + 2 * DK_C_BYTES + (unsigned)p.raw_bytes;
+    const unsigned stage_tx = DK_W_BYTES + (CTMA ? 2 * DK_C_BYTES : 0) + (unsigned)p.raw_bytes;
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t ctas = gridDim.x;
@@ -306,17 +309,21 @@ qmm_decode_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
         {
             if (lane == 0) {
                 asm volatile("prefetch.tensormap [%0];" ::"l"(&w_map) : "memory");
-                asm volatile("prefetch.tensormap [%0];" ::"l"(&s_map) : "memory");
-                asm volatile("prefetch.tensormap [%0];" ::"l"(&z_map) : "memory");
+                if constexpr (CTMA) {
+                    asm volatile("prefetch.tensormap [%0];" ::"l"(&s_map) : "memory");
+                    asm volatile("prefetch.tensormap [%0];" ::"l"(&z_map) : "memory");
+                }
                 asm volatile("prefetch.tensormap [%0];" ::"l"(&x_map) : "memory");
             }
             __syncwarp();
             auto load_weights = [&](int s, int rb, int kt) {
                 mbar_expect_tx_elect(full + s, stage_tx);
                 tma_load_2d(wst + (size_t)s * DK_W_BYTES, &w_map, kt * DK_WORDS, rb * DK_ROWS, full + s);
-                const int grp0 = ((kt * Geo::TILE_K) >> p.g_shift) & ~(DK_GBOX - 1);   // TMA boxes start on 16-byte boundaries
-                tma_load_2d(cst + (size_t)s * 2 * DK_C_BYTES, &s_map, grp0, rb * DK_ROWS, full + s);
-                tma_load_2d(cst + (size_t)s * 2 * DK_C_BYTES + DK_C_BYTES, &z_map, grp0, rb * DK_ROWS, full + s);
+                if constexpr (CTMA) {
+                    const int grp0 = ((kt * Geo::TILE_K) >> p.g_shift) & ~(DK_GBOX - 1);   // TMA boxes start on 16-byte boundaries
+                    tma_load_2d(cst + (size_t)s * 2 * DK_C_BYTES, &s_map, grp0, rb * DK_ROWS, full + s);
+                    tma_load_2d(cst + (size_t)s * 2 * DK_C_BYTES + DK_C_BYTES, &z_map, grp0, rb * DK_ROWS, full + s);
+                }
             };
             auto load_x = [&](int s, int kt) {
                 unsigned char *dst = rst + (size_t)s * p.raw_bytes;
@@ -553,14 +560,29 @@ qmm_decode_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
         // this lane's group inside the tile's box of scales / zero points (row pitch 16 bytes)
         const int goff = (4 * chunk * Geo::VPI) >> p.g_shift;
         const uint32_t c_off = (uint32_t)row_a * (DK_GBOX * 2) + (uint32_t)goff * 2;
-        auto make_const = [&](const unsigned char *cbox) {   // {scale, scale} and {1024 + zp, 1024 + zp}
+        auto make_const = [&](uint32_t sr, uint32_t zr) {    // {scale, scale} and {1024 + zp, 1024 + zp}
             GroupConst c;
-            const uint32_t sr = *reinterpret_cast<const unsigned short *>(cbox);
-            const uint32_t zr = *reinterpret_cast<const unsigned short *>(cbox + DK_C_BYTES);
             c.s2 = __byte_perm(sr, sr, 0x1010);
             c.z1024 = h2_as_u32(__hadd2(u32_as_h2(__byte_perm(zr, zr, 0x1010)), __float2half2_rn(1024.0f)));
             return c;
         };
+
+        auto box_const = [&](const unsigned char *cbox) {
+            return make_const(*reinterpret_cast<const unsigned short *>(cbox), *reinterpret_cast<const unsigned short *>(cbox + DK_C_BYTES));
+        };
+        // scale | zero point << 16 of this lane's chunk of the next tile in rows g and g + 8, when not by TMA
+        uint32_t sz_a = 0, sz_b = 0;
+        int rb = rb0;
+        auto load_consts = [&](int rbn, int ktn) {
+            if (ktn == p.KT) { ktn = 0; ++rbn; }
+            const int64_t G = p.K >> p.g_shift, grp = ((int64_t)ktn * Geo::TILE_K + 4 * chunk * Geo::VPI) >> p.g_shift;
+            const int64_t n = (int64_t)rbn * DK_ROWS + row_a;
+            const unsigned short *sp = reinterpret_cast<const unsigned short *>(p.scale), *zq = reinterpret_cast<const unsigned short *>(p.zp);
+            sz_a = sz_b = 0;                                // outside the matrix: the words there are zeros, too
+            if (grp < G && n < p.N) sz_a = (uint32_t)__ldg(sp + n * G + grp) | (uint32_t)__ldg(zq + n * G + grp) << 16;
+            if (grp < G && n + 8 < p.N) sz_b = (uint32_t)__ldg(sp + (n + 8) * G + grp) | (uint32_t)__ldg(zq + (n + 8) * G + grp) << 16;
+        };
+        if constexpr (!CTMA) load_consts(rb0, kt0);
 
         float acc[NACC][MT][4];
 #pragma unroll
@@ -578,11 +600,15 @@ qmm_decode_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
             mbar_wait(full + s, ph, dead, 2);               // packed words, scales, zero points
             mbar_wait(xdone + s, ph, dead, 6);              // activations converted
             Dequant<BITS> dqa, dqb;
-            {
+            if constexpr (CTMA) {
                 const int gtile = ((kt * Geo::TILE_K) >> p.g_shift) & (DK_GBOX - 1);   // the tile's first group inside its box
                 const unsigned char *cb = cst + (size_t)s * 2 * DK_C_BYTES + c_off + gtile * 2;
-                dqa.set(make_const(cb));
-                dqb.set(make_const(cb + 8 * DK_GBOX * 2));
+                dqa.set(box_const(cb));
+                dqb.set(box_const(cb + 8 * DK_GBOX * 2));
+            } else {
+                dqa.set(make_const(sz_a & 0xffffu, sz_a >> 16));
+                dqb.set(make_const(sz_b & 0xffffu, sz_b >> 16));
+                if (i + 1 < nt) load_consts(rb, kt + 1);
             }
             const unsigned char *wt = wst + (size_t)s * DK_W_BYTES + w_off;
             const uint4 wa = *reinterpret_cast<const uint4 *>(wt);
@@ -661,6 +687,7 @@ qmm_decode_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
                 if (lane == 0) mbar_arrive(red_full + b);
                 ++f;
                 kt = 0;
+                ++rb;
             } else {
                 ++kt;
             }
@@ -789,12 +816,12 @@ int launch_pdl(Kern kern, dim3 grid, dim3 block, size_t smem, int cluster, cudaS
 
 struct DecMaps { CUtensorMap w, s, z, x; };
 
-template <int BITS, int MT, bool EPI>
+template <int BITS, int MT, bool EPI, bool CTMA>
 int launch_dec(const DecMaps &maps, DecParams p, const Epilogue &ep, cudaStream_t st) {
-    auto kern = qmm_decode_kernel<BITS, MT, EPI>;
+    auto kern = qmm_decode_kernel<BITS, MT, EPI, CTMA>;
     constexpr size_t XB = DecX<BITS, MT>::BYTES;
     constexpr int NRED = MT == 4 ? 1 : 2;
-    const size_t stage = DK_W_BYTES + 2 * DK_C_BYTES + XB + (size_t)p.raw_bytes;
+    const size_t stage = DK_W_BYTES + (CTMA ? 2 * DK_C_BYTES : 0) + XB + (size_t)p.raw_bytes;
 
     int ctas = sm_count();
     if (ctas > DK_MAX_CTAS) ctas = DK_MAX_CTAS;
@@ -834,21 +861,19 @@ int launch_dec(const DecMaps &maps, DecParams p, const Epilogue &ep, cudaStream_
     return launch_pdl(kern, dim3((unsigned)ctas), dim3(DecWarps<MT>::THREADS), smem, p.cluster, st, maps.w, maps.s, maps.z, maps.x, p, ep);
 }
 
-template <int BITS>
-int launch_dec_mt(const DecMaps &maps, const DecParams &p, int mt, cudaStream_t st) {
-    const Epilogue ep = current_epilogue();
-    if (ep.act != BW_ACT_NONE || ep.residual) {
-        switch (mt) {
-            case 1: return launch_dec<BITS, 1, true>(maps, p, ep, st);
-            case 2: return launch_dec<BITS, 2, true>(maps, p, ep, st);
-            default: return launch_dec<BITS, 4, true>(maps, p, ep, st);
-        }
-    }
+template <int BITS, bool EPI>
+int launch_dec_mt(const DecMaps &maps, const DecParams &p, int mt, bool ctma, const Epilogue &ep, cudaStream_t st) {
     switch (mt) {
-        case 1: return launch_dec<BITS, 1, false>(maps, p, ep, st);
-        case 2: return launch_dec<BITS, 2, false>(maps, p, ep, st);
-        default: return launch_dec<BITS, 4, false>(maps, p, ep, st);
+        case 1: return launch_dec<BITS, 1, EPI, true>(maps, p, ep, st);      // (see dec_direct_consts)
+        case 2: return ctma ? launch_dec<BITS, 2, EPI, true>(maps, p, ep, st) : launch_dec<BITS, 2, EPI, false>(maps, p, ep, st);
+        default: return ctma ? launch_dec<BITS, 4, EPI, true>(maps, p, ep, st) : launch_dec<BITS, 4, EPI, false>(maps, p, ep, st);
     }
+}
+template <int BITS>
+int launch_dec_ep(const DecMaps &maps, const DecParams &p, int mt, bool ctma, cudaStream_t st) {
+    const Epilogue ep = current_epilogue();
+    return ep.act != BW_ACT_NONE || ep.residual ? launch_dec_mt<BITS, true>(maps, p, mt, ctma, ep, st)
+                                                : launch_dec_mt<BITS, false>(maps, p, mt, ctma, ep, st);
 }
 
 }  // namespace
@@ -867,9 +892,19 @@ int decode_device_status() {
     return v;
 }
 
+// Rows of scales and zero points that TMA can stride over (whole 16-byte units).
+static bool dec_const_tma(const void *scale, const void *zp, int64_t K, int g) {
+    return (K / g) % 8 == 0 && aligned_to(scale, 16) && aligned_to(zp, 16);
+}
+// Others are worth loading directly for more than 8 tokens and at least 2^22 weights; below either line the
+// cluster split-K kernel is as fast.  (4096 x 11008, W4 g128: 12.8 us there at 8 tokens against 13.1 for a shape
+// of that size here; 25.4 against 18.4 at 16 tokens, 30 against 22.8 at 32.  2048 x 1408 at 16 tokens: 6.7 there,
+// the fixed time of a launch here.)
+static bool dec_direct_consts(int64_t M, int64_t N, int64_t K) { return M > 8 && N * K >= (int64_t)1 << 22; }
+
 // Layout preconditions of the persistent decode kernel: at most 32 tokens, power-of-two groups
-// that hold a lane's 16-byte chunk (4 words), rows of packed words, scales, zero points and
-// activations that TMA can stride over (whole 16-byte units, 16-byte aligned bases).
+// that hold a lane's 16-byte chunk (4 words), rows of packed words and activations that TMA can stride
+// over (whole 16-byte units, 16-byte aligned bases).
 bool decode_path_ok(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, const int32_t *q,
                     const void *scale, const void *zp, int bits, int g) {
     if (!g_dec.enabled) return false;
@@ -882,7 +917,8 @@ bool decode_path_ok(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K,
     if (K > (int64_t)1 << 30 || N > (int64_t)DK_CNT_PER_WS * DK_ROWS) return false;
     if ((N + DK_ROWS - 1) / DK_ROWS * ((K / vpi + DK_WORDS - 1) / DK_WORDS) > (int64_t)1 << 30) return false;
     if (!aligned_to(q, 16)) return false;
-    if ((K / g) % 8 != 0 || !aligned_to(scale, 16) || !aligned_to(zp, 16)) return false;
+    // (the gated epilogue is only offered where scales and zero points come by TMA)
+    if (!dec_const_tma(scale, zp, K, g) && (!dec_direct_consts(M, N, K) || current_epilogue().act == BW_ACT_SILU_MUL)) return false;
     if (!aligned_to(x, 16) || (K * dtype_size(x_dtype)) % 16 != 0) return false;
     return encode_tiled_fn() != nullptr;
 }
@@ -903,7 +939,9 @@ int qmatmul_decode(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, 
     DecParams p = {};
     p.cnt = counter_slice(workspace);
     if (!p.cnt) return BW_ERR_UNSUPPORTED;
+    const bool ctma = dec_const_tma(scale, zp, K, g);
     p.part = reinterpret_cast<float *>(workspace);
+    p.scale = scale; p.zp = zp;
     p.bias = bias; p.out = out;
     p.M = M; p.N = N; p.K = K; p.x_dtype = x_dtype; p.out_dtype = out_dtype;
     int gs = 0;
@@ -921,18 +959,19 @@ int qmatmul_decode(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, 
     // boxes of 8*ceil(M/8) token slots x up to 256 k.  Everything outside a tensor arrives as zeros.
     int rc = encode_2d(&maps.w, CU_TENSOR_MAP_DATA_TYPE_INT32, q, (uint64_t)(K / vpi), (uint64_t)N, (uint64_t)(K / vpi) * 4,
                        DK_WORDS, DK_ROWS, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc == BW_OK) rc = encode_2d(&maps.s, CU_TENSOR_MAP_DATA_TYPE_UINT16, scale, (uint64_t)(K / g), (uint64_t)N, (uint64_t)(K / g) * 2,
+    if (!ctma) maps.s = maps.z = maps.w;                  // not used
+    if (rc == BW_OK && ctma) rc = encode_2d(&maps.s, CU_TENSOR_MAP_DATA_TYPE_UINT16, scale, (uint64_t)(K / g), (uint64_t)N, (uint64_t)(K / g) * 2,
                                     DK_GBOX, DK_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE);
-    if (rc == BW_OK) rc = encode_2d(&maps.z, CU_TENSOR_MAP_DATA_TYPE_UINT16, zp, (uint64_t)(K / g), (uint64_t)N, (uint64_t)(K / g) * 2,
+    if (rc == BW_OK && ctma) rc = encode_2d(&maps.z, CU_TENSOR_MAP_DATA_TYPE_UINT16, zp, (uint64_t)(K / g), (uint64_t)N, (uint64_t)(K / g) * 2,
                                     DK_GBOX, DK_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc == BW_OK) rc = encode_2d(&maps.x, x_dtype == BW_F32 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, x,
                                     (uint64_t)K, (uint64_t)M, (uint64_t)K * dtype_size(x_dtype),
                                     (uint32_t)(tile_k < DK_XBOX ? tile_k : DK_XBOX), (uint32_t)(mt * 8), CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc != BW_OK) return rc;
     switch (bits) {
-        case 2: rc = launch_dec_mt<2>(maps, p, mt, st); break;
-        case 4: rc = launch_dec_mt<4>(maps, p, mt, st); break;
-        default: rc = launch_dec_mt<8>(maps, p, mt, st); break;
+        case 2: rc = launch_dec_ep<2>(maps, p, mt, ctma, st); break;
+        case 4: rc = launch_dec_ep<4>(maps, p, mt, ctma, st); break;
+        default: rc = launch_dec_ep<8>(maps, p, mt, ctma, st); break;
     }
     if (rc == BW_OK) set_last_kernel("qmm_decode_kernel");
     return rc;

@@ -551,6 +551,33 @@ def test_persistent_decode_kernel_vs_oracle(case):
         assert_close_rms(as_f32(yb), as_f32(refb), 1e-2, str(case))
 
 
+@pytest.mark.parametrize("bits,g,N,K", [
+    # scales in rows of whole 16-byte units (TMA) or not; ragged last k-tiles and row blocks; clusters, whole row
+    # blocks, shares of several CTAs (N > 148 * 128); just below and above the line for direct scales
+    (4, 128, 384, 4096), (4, 32, 3300, 1312), (4, 128, 1000, 11008), (4, 64, 4000, 1088), (8, 16, 129, 640), (8, 128, 2978, 1408),
+    (8, 128, 2979, 1408), (2, 64, 2048, 2112), (2, 128, 500, 8576), (4, 128, 19200, 1152), (8, 32, 20000, 544),
+])
+def test_decode_kernel_matches_float64(bits, g, N, K):
+    gen = torch.Generator(device=DEV).manual_seed(N + K)
+    q = torch.randint(-2 ** 31, 2 ** 31 - 1, (N, K * bits // 32), generator=gen, device=DEV, dtype=torch.int32)
+    s = (torch.rand(N, K // g, generator=gen, device=DEV) * 0.02 + 0.001).half()
+    z = torch.randint(0, 2 ** bits, (N, K // g), generator=gen, device=DEV).half()
+    b = torch.randn(N, generator=gen, device=DEV).half()
+    w = dequantize_rtn(q, s, z, g, bits=bits).half().double()
+    for M in (1, 2, 8, 9, 16, 17, 32):
+        for xdt in (torch.float16, torch.bfloat16) if M != 17 else (torch.float32,):
+            x = torch.randn(M, K, generator=gen, device=DEV).to(xdt)
+            y = quantized_matmul_cuda(x, q, s, z, b if M % 2 else None, bits, g, out_dtype=torch.float32)
+            if xdt != torch.float32 and ((K // g) % 8 == 0 or (M > 8 and N * K >= 1 << 22)):
+                assert _lib.last_qmatmul_kernel() == "qmm_decode_kernel", (M, xdt)
+            xh = x.half().double()
+            ref = xh @ w.T + (b.double() if M % 2 else 0.0)
+            # fp32 sums: a few roundings of partial sums of the order of |x| . |W|
+            slack = 2.0 ** -23 * (K / 16 + 16) * (xh.abs() @ w.abs().T) + 1e-6
+            assert bool(((y.double() - ref).abs() <= slack).all()), (M, xdt, float((y.double() - ref).abs().max()))
+    assert _lib.lib().bw_device_status() == 0
+
+
 # --------------------------------------------------------------------------- backward
 
 @pytest.mark.parametrize("bits,g,gdt", [(4, 128, torch.float16), (8, 32, torch.float32), (2, 64, torch.bfloat16),
