@@ -21,20 +21,29 @@ def _compute_device(t):
     return torch.device("cuda", torch.cuda.current_device())
 
 
+def _resident(t, device):
+    """`t` without its graph, on `device`, contiguous: only the steps that it needs."""
+    t = t.detach()
+    if t.device != device:
+        t = t.to(device)
+    return t if t.is_contiguous() else t.contiguous()
+
+
 def _rtn_launch(weight, bits, group_size, scale_dtype, zp_dtype, upcast, flags=0):
     """weight: contiguous CUDA [N,K] float tensor.  Returns (q, scale, zp) on that device."""
     N, K = weight.shape
     vpi = 32 // bits
     G = K // group_size
-    q = torch.empty((N, K // vpi), dtype=torch.int32, device=weight.device)
-    scale = torch.empty((N, G), dtype=scale_dtype, device=weight.device)
-    zp = torch.empty((N, G), dtype=zp_dtype, device=weight.device)
+    dev = weight.device
+    q = torch.empty((N, K // vpi), dtype=torch.int32, device=dev)
+    scale = torch.empty((N, G), dtype=scale_dtype, device=dev)
+    zp = torch.empty((N, G), dtype=zp_dtype, device=dev)
     L = _lib.lib()
-    with torch.cuda.device(weight.device):
-        rc = L.bw_rtn_quantize_pack(_lib.ptr(weight), _lib.dtype_code(weight.dtype), N, K, bits, group_size,
-                                    _lib.ptr(q), _lib.ptr(scale), _lib.dtype_code(scale_dtype),
-                                    _lib.ptr(zp), _lib.dtype_code(zp_dtype),
-                                    (_lib.RTN_UPCAST_F32 if upcast else 0) | flags, _lib.stream_ptr(weight.device))
+    with _lib.on_device(dev):
+        rc = L.bw_rtn_quantize_pack(weight.data_ptr(), _lib.dtype_code(weight.dtype), N, K, bits, group_size,
+                                    q.data_ptr(), scale.data_ptr(), _lib.dtype_code(scale_dtype),
+                                    zp.data_ptr(), _lib.dtype_code(zp_dtype),
+                                    (_lib.RTN_UPCAST_F32 if upcast else 0) | flags, _lib.raw_stream(dev))
     _lib.check(rc)
     return q, scale, zp
 
@@ -54,7 +63,6 @@ def _validate(weight, bits, group_size):
         raise RuntimeError(f"in_features={in_features} is not a multiple of {32 // bits} codes per int32")
 
 
-@torch.no_grad()
 def quantize_rtn(weight: torch.Tensor, bits: int = 8, group_size: int = 32):
     """Drop-in for bitween/functional.py:3-45.
 
@@ -66,7 +74,7 @@ def quantize_rtn(weight: torch.Tensor, bits: int = 8, group_size: int = 32):
     if weight.dtype not in _FLOAT_DTYPES:
         raise TypeError(f"quantize_rtn: unsupported weight dtype {weight.dtype} (float32/float16/bfloat16)")
     src_device = weight.device
-    w = weight.detach().to(_compute_device(weight)).contiguous()
+    w = _resident(weight, _compute_device(weight))
     q, scale, zp = _rtn_launch(w, bits, group_size, weight.dtype, torch.int32, upcast=False)
     if not src_device.type == "cuda":
         q, scale, zp = q.to(src_device), scale.to(src_device), zp.to(src_device)
@@ -128,7 +136,6 @@ def quantize_rtn_many_to_module_buffers(weights, bits: int, group_size: int):
     return results
 
 
-@torch.no_grad()
 def dequantize_rtn(q_packed: torch.Tensor, scale: torch.Tensor, zero_point: torch.Tensor, group_size: int,
                    bits: int = 8, out_dtype: torch.dtype = torch.float32):
     """Drop-in for bitween/functional.py:47-71: float32 [N, K] = scale * (code - zero_point).
@@ -145,18 +152,18 @@ def dequantize_rtn(q_packed: torch.Tensor, scale: torch.Tensor, zero_point: torc
     G = K // group_size
     src_device = q_packed.device
     dev = _compute_device(q_packed)
-    q = q_packed.detach().to(dev).contiguous()
-    s = scale.detach().to(dev).reshape(N, G).contiguous()
-    z = zero_point.detach().to(dev).reshape(N, G).contiguous()
+    q = _resident(q_packed, dev)
+    s = _resident(scale.reshape(N, G), dev)
+    z = _resident(zero_point.reshape(N, G), dev)
     if s.dtype not in _FLOAT_DTYPES:
         s = s.to(torch.float32)
     if z.dtype not in _FLOAT_DTYPES and z.dtype != torch.int32:
         z = z.to(torch.int32) if not z.dtype.is_floating_point else z.to(torch.float32)
     out = torch.empty((N, K), dtype=out_dtype, device=dev)
     L = _lib.lib()
-    with torch.cuda.device(dev):
-        rc = L.bw_dequantize(_lib.ptr(q), _lib.ptr(s), _lib.dtype_code(s.dtype), _lib.ptr(z),
-                             _lib.dtype_code(z.dtype), N, K, bits, group_size, _lib.ptr(out),
-                             _lib.dtype_code(out_dtype), _lib.stream_ptr(dev))
+    with _lib.on_device(dev):
+        rc = L.bw_dequantize(q.data_ptr(), s.data_ptr(), _lib.dtype_code(s.dtype), z.data_ptr(),
+                             _lib.dtype_code(z.dtype), N, K, bits, group_size, out.data_ptr(),
+                             _lib.dtype_code(out_dtype), _lib.raw_stream(dev))
     _lib.check(rc)
     return out if src_device.type == "cuda" else out.to(src_device)

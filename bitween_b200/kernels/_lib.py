@@ -4,6 +4,7 @@ This is the only place the Python host code crosses into native code.  There is 
 fallback of any kind: if the shared library is missing (and cannot be built because nvcc
 is absent) or no CUDA device is present, the calls raise.
 """
+import contextlib
 import ctypes
 import os
 import threading
@@ -161,6 +162,14 @@ def stream_ptr(device):
 def raw_stream(device):
     """The current stream of `device` as an integer handle."""
     return torch._C._cuda_getCurrentRawStream(device.index)
+
+
+_NO_GUARD = contextlib.nullcontext()
+
+
+def on_device(device):
+    """Context in which `device` is the current one; nothing is switched when it already is."""
+    return _NO_GUARD if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def ptr(t):
