@@ -233,7 +233,8 @@ int launch_v(const void *w, int64_t N, int64_t K, int bits, int g, const float *
 // The per-group parameters of a tuned layer (bitween/wrapper.py:127-140) from the group extrema of the frozen
 // weight and the learnable factors, and their backward: a handful of operations per group, one launch each
 // instead of one per operation (7 forward, 13 backward: at 32 groups a row they cost more than the pass over
-// the weights).  One rounding per operation, in torch's order; the quotients are correctly rounded.
+// the weights).  One rounding per operation, in torch's order; the quotients are correctly rounded.  4096 x 4096,
+// g 128: 2.4 us forward and 3.5 us backward; the whole training step at 256 tokens 445 us instead of 543.
 template <typename T>
 __global__ void __launch_bounds__(256)
 group_params_kernel(const T *__restrict__ w_min, const T *__restrict__ w_max, const float *__restrict__ min_scale,
