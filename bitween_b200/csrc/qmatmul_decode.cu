@@ -31,6 +31,7 @@
 // CTA stops waiting.
 #include <cuda.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "bw_common.cuh"
@@ -60,17 +61,18 @@ constexpr int DK_MAX_CTAS = 160;                   // upper bound of the grid (s
 constexpr int DK_MAX_STAGES = 12;
 constexpr int DK_XBOX = 256;                       // widest TMA box of raw activations (elements)
 constexpr unsigned DK_WAIT_LIMIT = 1u << 22;       // polls of >= 20 ns each
-constexpr int DK_CNT_PER_WS = 4096;                // row-block counters per registered workspace
-constexpr int DK_CNT_WS = 64;                      // workspaces per device that can use the kernel at a time
+constexpr int DK_CNT_PER_WS = 4096;                // row-block counters per slice
+constexpr int DK_CNT_WS = 64;                      // slices for calls outside captures: one per workspace in use at a time
+constexpr int DK_CNT_GRAPHS = 448;                 // slices for captured calls: one per live graph and captured stream
 
 __device__ int g_dec_status = 0;
 // Arrival counters of the row blocks.  atomicInc wraps them back to 0 when the last share of a
 // row block arrives, so a completed call leaves them ready for the next one; they live here,
 // not in the caller's scratch, because they must be zero before the first call.
-__device__ unsigned g_dec_cnt[DK_CNT_WS * DK_CNT_PER_WS];
+__device__ unsigned g_dec_cnt[(DK_CNT_WS + DK_CNT_GRAPHS) * DK_CNT_PER_WS];
 
 struct DecParams {
-    unsigned *cnt;        // this call's slice of g_dec_cnt
+    unsigned *cnt;        // this call's slice of g_dec_cnt; null when no row block is shared through the scratch
     float *part;          // partial tiles [2 * cta + which][MTOK][128] fp32
     const __half *bias;
     const __half *scale, *zp;   // read directly when they do not come by TMA
@@ -748,26 +750,75 @@ int sm_count() {
 
 }  // namespace
 
-// The slice of g_dec_cnt that calls with this workspace use.  Calls that may overlap on the GPU
-// already need distinct workspaces, so they also get distinct counters.  Slices are handed out
-// per workspace address; when all are taken the least recently used one is reassigned (a call
-// leaves its counters at zero, so a slice can change hands as long as no kernel of its previous
-// owner is still running -- that would take more than DK_CNT_WS workspaces with work in flight
+static unsigned *counter_base(int dev) {
+    static std::atomic<unsigned *> base[64];
+    unsigned *p = base[dev].load(std::memory_order_acquire);
+    if (!p) {
+        void *v = nullptr;
+        if (cudaGetSymbolAddress(&v, g_dec_cnt) != cudaSuccess) return nullptr;
+        p = reinterpret_cast<unsigned *>(v);
+        base[dev].store(p, std::memory_order_release);
+    }
+    return p;
+}
+
+// The slice of g_dec_cnt that a captured call uses.  A graph may be replayed at any time beside other graphs
+// and beside calls outside of graphs, whatever workspace they were given, so it owns its slices: one per stream
+// of the capture (calls of one stream follow each other in the graph as well).  The graph holds a user object
+// that gives the slice back when it and everything instantiated from it are gone and no launch is running.
+static unsigned *graph_counter_slice(int dev, cudaStream_t st, cudaGraph_t graph, unsigned long long capture) {
+    struct Slot { std::atomic<int> taken; unsigned long long capture; cudaStream_t stream; };
+    static Slot slots[64][DK_CNT_GRAPHS];
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    unsigned *base = counter_base(dev) + (size_t)DK_CNT_WS * DK_CNT_PER_WS;
+    int pick = -1;
+    for (int i = 0; i < DK_CNT_GRAPHS; ++i) {
+        Slot &s = slots[dev][i];
+        if (!s.taken.load(std::memory_order_acquire)) { if (pick < 0) pick = i; continue; }
+        if (s.capture == capture && s.stream == st) return base + (size_t)i * DK_CNT_PER_WS;
+    }
+    if (pick < 0) return nullptr;
+    Slot &s = slots[dev][pick];
+    cudaUserObject_t obj = nullptr;
+    // (the destructor runs on a thread of the driver and may not call CUDA: it only marks the slot)
+    if (cudaUserObjectCreate(&obj, &s, [](void *v) { static_cast<Slot *>(v)->taken.store(0, std::memory_order_release); }, 1,
+                             cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    s.capture = capture; s.stream = st;
+    s.taken.store(1, std::memory_order_release);
+    if (cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        (void)cudaGetLastError();
+        (void)cudaUserObjectRelease(obj, 1);              // runs the destructor
+        return nullptr;
+    }
+    return base + (size_t)pick * DK_CNT_PER_WS;
+}
+
+// The slice of g_dec_cnt that a call on `st` with this workspace uses; null when a capture finds none free.
+// Outside captures, calls that may overlap on the GPU already need distinct workspaces, so they also get
+// distinct counters.  Slices are handed out per workspace address; when all are taken the least recently used
+// one is reassigned (a call leaves its counters at zero, so a slice can change hands as long as no kernel of its
+// previous owner is still running -- that would take more than DK_CNT_WS workspaces with work in flight
 // on one device at a time).
-unsigned *counter_slice(const void *workspace) {
+static unsigned *counter_slice(const void *workspace, int dev, cudaStream_t st) {
+    if (st != nullptr && st != cudaStreamLegacy) {        // (the legacy stream cannot be captured)
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        unsigned long long capture = 0;
+        cudaGraph_t graph = nullptr;
+        if (cudaStreamGetCaptureInfo(st, &status, &capture, &graph, nullptr, nullptr) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+        if (status == cudaStreamCaptureStatusActive) return graph_counter_slice(dev, st, graph, capture);
+    }
     static std::mutex mu;
     static const void *owner[64][DK_CNT_WS] = {};
     static unsigned long long used[64][DK_CNT_WS] = {};
     static unsigned long long tick = 0;
-    static unsigned *base[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
     std::lock_guard<std::mutex> lock(mu);
-    if (!base[dev]) {
-        void *p = nullptr;
-        if (cudaGetSymbolAddress(&p, g_dec_cnt) != cudaSuccess) return nullptr;
-        base[dev] = reinterpret_cast<unsigned *>(p);
-    }
     int pick = -1;
     for (int i = 0; i < DK_CNT_WS; ++i) {
         if (owner[dev][i] == workspace) { pick = i; break; }
@@ -780,7 +831,7 @@ unsigned *counter_slice(const void *workspace) {
     }
     owner[dev][pick] = workspace;
     used[dev][pick] = ++tick;
-    return base[dev] + (size_t)pick * DK_CNT_PER_WS;
+    return counter_base(dev) + (size_t)pick * DK_CNT_PER_WS;
 }
 
 namespace {
@@ -823,7 +874,11 @@ int launch_dec(const DecMaps &maps, DecParams p, const Epilogue &ep, cudaStream_
     constexpr int NRED = MT == 4 ? 1 : 2;
     const size_t stage = DK_W_BYTES + (CTMA ? 2 * DK_C_BYTES : 0) + XB + (size_t)p.raw_bytes;
 
+    int dev = 0;
+    BW_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !counter_base(dev)) return BW_ERR_UNSUPPORTED;   // (looked up by the first call, whatever its shape)
     int ctas = sm_count();
+    bool shared = true;                                   // CTAs may share a row block through the scratch
     if (ctas > DK_MAX_CTAS) ctas = DK_MAX_CTAS;
     if (g_dec.max_ctas > 0) {
         if (ctas > g_dec.max_ctas) ctas = g_dec.max_ctas;
@@ -834,6 +889,7 @@ int launch_dec(const DecMaps &maps, DecParams p, const Epilogue &ep, cudaStream_
         int per_rb = 1;
         while (per_rb * 2 <= 8 && p.RB * per_rb * 2 <= ctas && per_rb * 2 <= p.KT) per_rb *= 2;
         ctas = p.RB * per_rb;
+        shared = false;
         p.cluster = per_rb;
         p.cluster_leader = (size_t)(per_rb - 1) * MT * 8 * DK_ROWS * 4 <= 32 * 1024 ? 1 : 0;
     }
@@ -844,6 +900,15 @@ int launch_dec(const DecMaps &maps, DecParams p, const Epilogue &ep, cudaStream_
                          16 + DK_MAX_CTAS * 4 + cpart_bytes + 64;
     const size_t budget = (size_t)(g_dec.smem_kb > 0 ? g_dec.smem_kb : 224) * 1024;
     if (budget < fixed + 2 * stage) return BW_ERR_UNSUPPORTED;
+    if (shared) {
+        p.cnt = counter_slice(p.part, dev, st);
+        if (!p.cnt) {
+            // no slice for this capture: the caller has another kernel, except for the gated epilogue, which
+            // then gives every CTA whole row blocks
+            if (ep.act != BW_ACT_SILU_MUL) return BW_ERR_UNSUPPORTED;
+            while (p.RB % ctas) --ctas;
+        }
+    }
     int stages = (int)((budget - fixed) / stage);
     const int per_cta = (p.tiles + ctas - 1) / ctas;
     if (stages > per_cta) stages = per_cta;           // a ring deeper than the CTA's tile count is never filled
@@ -852,11 +917,9 @@ int launch_dec(const DecMaps &maps, DecParams p, const Epilogue &ep, cudaStream_
     p.stages = stages;
     const size_t smem = fixed + (size_t)stages * stage;
     static size_t configured[64] = {};   // per instantiation and device; grows monotonically
-    int dev = 0;
-    BW_CUDA_TRY(cudaGetDevice(&dev));
-    if (smem > 48 * 1024 && (dev < 0 || dev >= 64 || smem > configured[dev])) {
+    if (smem > 48 * 1024 && smem > configured[dev]) {
         BW_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (dev >= 0 && dev < 64) configured[dev] = smem;
+        configured[dev] = smem;
     }
     return launch_pdl(kern, dim3((unsigned)ctas), dim3(DecWarps<MT>::THREADS), smem, p.cluster, st, maps.w, maps.s, maps.z, maps.x, p, ep);
 }
@@ -887,7 +950,7 @@ int decode_device_status() {
         // a CTA that gave up may have left row-block counters half way: clear them all
         (void)cudaMemcpyToSymbol(g_dec_status, &zero, sizeof(int));
         void *cnt = nullptr;
-        if (cudaGetSymbolAddress(&cnt, g_dec_cnt) == cudaSuccess) (void)cudaMemset(cnt, 0, sizeof(unsigned) * DK_CNT_WS * DK_CNT_PER_WS);
+        if (cudaGetSymbolAddress(&cnt, g_dec_cnt) == cudaSuccess) (void)cudaMemset(cnt, 0, sizeof(g_dec_cnt));
     }
     return v;
 }
@@ -929,7 +992,8 @@ size_t decode_workspace_bytes(int64_t M, int64_t N, int64_t K, int bits) {
     return (size_t)2 * DK_MAX_CTAS * dec_token_tiles(M) * 8 * DK_ROWS * sizeof(float);
 }
 
-// Returns BW_ERR_UNSUPPORTED (nothing launched) when no ring of two stages fits; the caller then uses the cluster split-K kernel.
+// Returns BW_ERR_UNSUPPORTED (nothing launched) when no ring of two stages fits or no counters are free; the caller
+// then uses the cluster split-K kernel.
 int qmatmul_decode(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, const int32_t *q,
                    const __half *scale, const __half *zp, const __half *bias, void *out, int out_dtype,
                    int bits, int g, void *workspace, cudaStream_t st) {
@@ -937,8 +1001,6 @@ int qmatmul_decode(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, 
     const int vpi = 32 / bits, mt = dec_token_tiles(M);
     const int tile_k = DK_WORDS * vpi;
     DecParams p = {};
-    p.cnt = counter_slice(workspace);
-    if (!p.cnt) return BW_ERR_UNSUPPORTED;
     const bool ctma = dec_const_tma(scale, zp, K, g);
     p.part = reinterpret_cast<float *>(workspace);
     p.scale = scale; p.zp = zp;

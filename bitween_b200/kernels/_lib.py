@@ -177,29 +177,36 @@ def ptr(t):
 
 
 _workspaces = {}
-_retired = []
+
+
+def _capturing(raw_stream):
+    # (the default stream, handle 0, cannot be captured)
+    return raw_stream != 0 and torch.cuda.is_current_stream_capturing()
 
 
 def workspace(device, nbytes):
-    """Caller-owned scratch for bw_qmatmul, cached per (device, stream): calls that may overlap on
-    the GPU must not share scratch, and calls on one stream are ordered.  The buffer only grows;
-    it is never freed while the process lives, so pointers captured in CUDA graphs stay valid
-    as long as the first capture already saw the largest size it needs."""
+    """Scratch for one bw_qmatmul call on the current stream of `device` (the current device).
+
+    Outside captures it is cached per (device, stream) and only grows: calls that may overlap on the GPU must not
+    share scratch, and calls on one stream are ordered.  A captured call takes scratch of its own from the graph's
+    memory pool instead: torch captures every graph on the same stream, but graphs are replayed on any."""
     if nbytes == 0:
         return None
-    key = (device.index, raw_stream(device))
+    stream = raw_stream(device)
+    if _capturing(stream):
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    key = (device.index, stream)
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
-        if buf is not None:
-            _retired.append(buf)   # a captured CUDA graph may still hold its address
         buf = torch.empty(max(nbytes, 1 << 21), dtype=torch.uint8, device=device)
         _workspaces[key] = buf
     return buf
 
 
 def current_workspace(device, raw_stream):
-    """The scratch `workspace` would return on this stream if it is large enough; None before the first call."""
-    return _workspaces.get((device.index, raw_stream))
+    """The scratch `workspace` would return on this stream if it is large enough; None before the first call
+    and inside a capture."""
+    return None if _capturing(raw_stream) else _workspaces.get((device.index, raw_stream))
 
 
 def last_qmatmul_kernel():

@@ -139,12 +139,14 @@ BW_API int bw_dequantize(const int32_t *qweight, const void *scale, int scale_dt
  *                   (bitween/modules.py:97,101); BW_BF16: bf16(acc + bias);
  *                   BW_F32: acc + bias with no 16-bit rounding (fp32-accumulate checks)
  *   workspace       device scratch of at least bw_qmatmul_workspace_bytes(...) bytes, or
- *                   NULL when that is 0.  Calls that overlap on the GPU must not share it,
- *                   and a workspace address identifies the caller to the library (the
- *                   decode kernel keeps its row-block counters per workspace address, for
- *                   up to 64 addresses per device; further ones use the cluster kernel).
- *                   Make the first call with a new workspace address outside a stream
- *                   capture (it looks up the address of the library's counter array).
+ *                   NULL when that is 0.  Calls that overlap on the GPU must not share it;
+ *                   a call captured into a CUDA graph runs whenever the graph is replayed,
+ *                   so graphs that may be replayed beside each other need a workspace each.
+ *                   The decode kernel's row-block counters are the library's: outside
+ *                   captures they go by workspace address (up to 64 with work in flight per
+ *                   device), a captured graph owns its own until it is destroyed (beyond 448
+ *                   live graphs the cluster kernel runs).  Make the first call on a device
+ *                   outside a stream capture (it looks up the address of the counters).
  * Accumulation is fp32.  The kernel is chosen from M and the layout: up to 32 tokens run on
  * the persistent TMA-fed decode kernel (one launch; needs K/group_size to be a multiple of 8
  * and 16-byte aligned rows, else the cluster split-K streaming kernel runs), more on the

@@ -230,3 +230,23 @@ def test_wrapper_linear_host_logic_with_oracle_doubles(monkeypatch):
     want_q, want_s, want_z = oracle.quantize_rtn(to_np(wl.orig_weight), oracle.F32, 4, 32)
     assert np.array_equal(to_np(ql.qweight), want_q)
     assert wrapper.unified_unwrapper(wl, apply_quantization=False) is wl.orig_layer
+
+
+def test_captured_calls_get_scratch_of_their_own(monkeypatch):
+    # torch.cuda.graph captures every graph on the same stream: scratch cached per stream would be shared by graphs
+    # that are replayed beside each other
+    from bitween_b200.kernels import _lib
+    dev = torch.device("cpu")
+    monkeypatch.setattr(_lib, "_workspaces", {})
+    monkeypatch.setattr(_lib, "raw_stream", lambda device: 7)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    eager = _lib.workspace(dev, 4096)
+    assert _lib.workspace(dev, 1024) is eager and _lib.current_workspace(dev, 7) is eager
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    assert _lib.current_workspace(dev, 7) is None
+    first, second = _lib.workspace(dev, 4096), _lib.workspace(dev, 4096)
+    assert len({t.data_ptr() for t in (eager, first, second)}) == 3
+    assert list(_lib._workspaces.values()) == [eager]
+    # the default stream cannot be captured: what another thread captures does not matter
+    monkeypatch.setattr(_lib, "raw_stream", lambda device: 0)
+    assert _lib.workspace(dev, 4096) is _lib.workspace(dev, 4096) is _lib.current_workspace(dev, 0)
