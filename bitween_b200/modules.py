@@ -73,11 +73,12 @@ class QuantizedLinear(nn.Module):
             self.bias = None
 
     def forward(self, x):
-        # extension: set layer.out_dtype = torch.bfloat16.  (Looked up in the places an attribute can be in
-        # before asking nn.Module, whose answer to a missing name is an exception.)
-        out_dtype = None
-        if "out_dtype" in self.__dict__ or hasattr(type(self), "out_dtype"):
-            out_dtype = self.out_dtype
+        # extension: set layer.out_dtype = torch.bfloat16.  (Where only nn.Module's own look-up is left, whose answer
+        # to a missing name is an exception, it is not asked.)
+        out_dtype, cls = None, type(self)
+        if "out_dtype" in self.__dict__ or hasattr(cls, "out_dtype") or cls.__getattr__ is not nn.Module.__getattr__ \
+                or cls.__getattribute__ is not nn.Module.__getattribute__:
+            out_dtype = getattr(self, "out_dtype", None)
         if out_dtype is None:
             return QuantizedLinearFunction.apply(x, self.qweight, self.scale, self.zero_point, self.bias,
                                                  self.bits, self.group_size)

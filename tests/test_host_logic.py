@@ -250,3 +250,30 @@ def test_captured_calls_get_scratch_of_their_own(monkeypatch):
     # the default stream cannot be captured: what another thread captures does not matter
     monkeypatch.setattr(_lib, "raw_stream", lambda device: 0)
     assert _lib.workspace(dev, 4096) is _lib.workspace(dev, 4096) is _lib.current_workspace(dev, 0)
+
+
+def test_out_dtype_is_found_wherever_a_subclass_keeps_it(monkeypatch):
+    seen = []
+    monkeypatch.setattr(modules.QuantizedLinearFunction, "apply", lambda *args: seen.append(args[7:]))
+
+    class ByGetattr(QuantizedLinear):
+        def __getattr__(self, name):
+            return torch.bfloat16 if name == "out_dtype" else super().__getattr__(name)
+
+    class ByProperty(QuantizedLinear):
+        out_dtype = property(lambda self: torch.float32)
+
+    class ByGetattribute(QuantizedLinear):
+        def __getattribute__(self, name):
+            return torch.float32 if name == "out_dtype" else super().__getattribute__(name)
+
+    x = torch.zeros(1, 64)
+    for cls, want in ((QuantizedLinear, ()), (ByGetattr, (torch.bfloat16,)), (ByProperty, (torch.float32,)),
+                      (ByGetattribute, (torch.float32,))):
+        layer = cls(64, 8, bits=4, group_size=32)
+        layer(x)
+        assert seen.pop() == want, cls
+        if cls is QuantizedLinear:
+            layer.out_dtype = torch.bfloat16
+            layer(x)
+            assert seen.pop() == (torch.bfloat16,)
