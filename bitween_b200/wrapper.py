@@ -238,9 +238,10 @@ class WrapperLinear(nn.Module):
 
     def _fused_group_params(self):
         """`_group_params` by one kernel where its operands are what the constructor made them; None otherwise
-        (no factors, a module cast to another dtype, a subclass with parameters of its own)."""
+        (no factors, a module cast to another dtype, `_group_params` replaced in a subclass, on the class or on the
+        instance)."""
         lo, hi, a, b = self._w_min, self._w_max, self.min_scale, self.max_scale
-        if a is None or b is None or type(self)._group_params is not WrapperLinear._group_params:
+        if a is None or b is None or getattr(self._group_params, "__func__", None) is not _GROUP_PARAMS:
             return None
         for t in (lo, hi, a, b):
             if type(t) not in (torch.Tensor, nn.Parameter) or not t.is_cuda or not t.is_contiguous() or t.shape != lo.shape or t.device != lo.device:
@@ -291,6 +292,9 @@ class WrapperLinear(nn.Module):
             if self.orig_layer.bias is not None:
                 q_layer.bias.copy_(self.orig_layer.bias)
             return q_layer
+
+
+_GROUP_PARAMS = WrapperLinear._group_params      # the operations that the kernels stand for
 
 
 def _get_module(model, module_name: str):

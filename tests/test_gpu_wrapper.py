@@ -261,3 +261,17 @@ def test_group_parameter_kernels_equal_the_separate_operations(dt, bits, N, G):
     assert WrapperLinear(layer, bits=bits, group_size=g, enable_minmax_tuning=False)._fused_group_params() is None
     assert WrapperLinear(layer, bits=bits, group_size=g).half()._fused_group_params() is None
     assert type("Own", (WrapperLinear,), {"_group_params": lambda self: None})(layer, bits=bits, group_size=g)._fused_group_params() is None
+
+
+def test_group_parameters_replaced_on_the_instance_or_the_class_are_used(monkeypatch):
+    layer = torch.nn.Linear(64, 8, bias=False, device=DEV)
+    x = torch.randn(3, 64, device=DEV)
+    scale, zp = torch.full((8, 4), 0.125, device=DEV), torch.full((8, 4), 3.0, device=DEV)
+    want = torch.nn.functional.linear(x, fake_quantize(layer.weight.data, scale, zp, torch.zeros(8, 64, device=DEV), 4, 16)[0])
+    wl = WrapperLinear(layer, bits=4, group_size=16)
+    assert not torch.equal(wl(x), want)
+    wl._group_params = lambda: (scale, zp)
+    assert torch.equal(wl(x), want)
+    other = WrapperLinear(layer, bits=4, group_size=16)
+    monkeypatch.setattr(WrapperLinear, "_group_params", lambda self: (scale, zp))
+    assert torch.equal(other(x), want)
