@@ -132,6 +132,13 @@ class _GroupParams(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_scale, grad_zero_point):
         w_min, w_max, scale, zero_point, span = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            # create_graph: the kernel's operations one by one, so that the gradients can be differentiated
+            qmax = torch.full((), (1 << ctx.bits) - 1, dtype=span.dtype, device=span.device)
+            g_lo = -(grad_zero_point / scale)
+            g_scale = grad_scale - grad_zero_point * (zero_point / scale)
+            g_span = torch.where(span / qmax >= 1e-8, g_scale, 0.0) / qmax
+            return None, None, (g_lo - g_span) * w_min, g_span * w_max, None
         gs, gz = grad_scale.contiguous(), grad_zero_point.contiguous()
         g_min = torch.empty_like(scale)
         g_max = torch.empty_like(scale)

@@ -275,3 +275,26 @@ def test_group_parameters_replaced_on_the_instance_or_the_class_are_used(monkeyp
     other = WrapperLinear(layer, bits=4, group_size=16)
     monkeypatch.setattr(WrapperLinear, "_group_params", lambda self: (scale, zp))
     assert torch.equal(other(x), want)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16], ids=str)
+def test_gradients_of_the_factors_can_be_differentiated(dt):
+    # create_graph: the same gradients as without a graph, and the second derivatives of the separate operations
+    layer = torch.nn.Linear(128, 24, bias=False, device=DEV, dtype=dt)
+    wl = WrapperLinear(layer, bits=4, group_size=16)
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    with torch.no_grad():
+        for t in (wl.min_scale, wl.max_scale):
+            t.copy_(torch.rand(24, 8, generator=gen, device=DEV) * 0.2 + 0.9)
+    factors = (wl.min_scale, wl.max_scale)
+    gs, gz, u, v = (torch.randn(24, 8, generator=gen, device=DEV) for _ in range(4))
+    second = []
+    for params in (wl._fused_group_params, wl._group_params):
+        gs_, gz_ = gs.clone().requires_grad_(True), gz.clone().requires_grad_(True)
+        first = torch.autograd.grad(params(), factors, (gs_, gz_), create_graph=True)
+        plain = torch.autograd.grad(params(), factors, (gs, gz))
+        for a, b in zip(first, plain):
+            assert torch.allclose(a, b, rtol=2.0 ** -20, atol=0)       # a few roundings of no more than two terms
+        second.append(torch.autograd.grad((first[0] * u + first[1] * v).sum(), (*factors, gs_, gz_)))
+    for a, b in zip(*second):
+        assert torch.allclose(a, b, rtol=1e-5, atol=1e-6 * float(b.abs().max()))
