@@ -836,6 +836,11 @@ static unsigned *counter_slice(const void *workspace, int dev, cudaStream_t st) 
 
 namespace {
 
+inline int dec_ctas_per_block(int64_t RB, int64_t KT, int ctas) {
+    int n = 1;
+    while (n * 2 <= 8 && RB * n * 2 <= ctas && n * 2 <= KT) n *= 2;
+    return n;
+}
 inline int dec_token_tiles(int64_t M) { return M <= 8 ? 1 : (M <= 16 ? 2 : 4); }
 
 template <typename Kern, typename... Args>
@@ -886,8 +891,7 @@ int launch_dec(const DecMaps &maps, DecParams p, const Epilogue &ep, cudaStream_
         // no more row blocks than SMs: give each row block the same number of CTAs, 1, 2, 4 or 8,
         // launched as one thread-block cluster that adds its shares through distributed shared
         // memory (no round trips through L2)
-        int per_rb = 1;
-        while (per_rb * 2 <= 8 && p.RB * per_rb * 2 <= ctas && per_rb * 2 <= p.KT) per_rb *= 2;
+        const int per_rb = dec_ctas_per_block(p.RB, p.KT, ctas);
         ctas = p.RB * per_rb;
         shared = false;
         p.cluster = per_rb;
@@ -959,11 +963,32 @@ int decode_device_status() {
 static bool dec_const_tma(const void *scale, const void *zp, int64_t K, int g) {
     return (K / g) % 8 == 0 && aligned_to(scale, 16) && aligned_to(zp, 16);
 }
-// Others are worth loading directly for more than 8 tokens and at least 2^22 weights; below either line the
-// cluster split-K kernel is as fast.  (4096 x 11008, W4 g128: 12.8 us there at 8 tokens against 13.1 for a shape
-// of that size here; 25.4 against 18.4 at 16 tokens, 30 against 22.8 at 32.  2048 x 1408 at 16 tokens: 6.7 there,
-// the fixed time of a launch here.)
-static bool dec_direct_consts(int64_t M, int64_t N, int64_t K) { return M > 8 && N * K >= (int64_t)1 << 22; }
+// Others are loaded directly where that beats the cluster split-K kernel, from 9 tokens and 2^22 weights on.  Measured
+// over 770 random layers of 512..32768 rows and 1024..30000 columns (2 / 4 / 8 bits, groups of 32..128, 9..32 tokens,
+// weights not in L2); below, us there / here:
+//   * the grid has to be resident at once; the chip holds 33 clusters of 4 and 15 of 8.  2048 x 8448, W4, 16 clusters of 8,
+//     14 tokens: 10.9 / 21.0;
+//   * idle SMs cost more here: 5248 x 25472, W8, 82 CTAs, 22 tokens: 106 / 132; 4096 x 9856, W4, 128 CTAs, 12 tokens:
+//     22.7 / 17.6.  Above 16 tokens the other kernel has two blocks a SM only, and at 2 and 4 bits this one wins from
+//     64 CTAs on: 5888 x 9024, W4, 92 CTAs, 29 tokens: 42.7 / 33.8;
+//   * a launch costs a fixed 6-8 us, which needs a few tiles a CTA: 11392 x 1280, W2, 3 tiles, 25 tokens: 10.1 / 13.0;
+//   * shares through the scratch (more row blocks than SMs) add 3-5 us: 30720 x 1536, W4, 22 tokens: 19.1 / 26.4;
+//     22912 x 5568: 70.2 / 54.8;
+//   * the other kernel cuts a row into 8 pieces at most: 768 x 21760, W4, 20 tokens: 34.4 / 21.8, whatever the grid.
+// In sum over all 1545 calls 0.84 of the other kernel's time (0.87 if all were taken, 0.82 for the better one each
+// time); 19 calls lose more than 8 %, none more than 19 %.
+static bool dec_direct_consts(int64_t M, int64_t N, int64_t K, int bits) {
+    if (M <= 8 || N * K < (int64_t)1 << 22) return false;
+    constexpr int64_t SMS = 148;
+    const int64_t RB = (N + DK_ROWS - 1) / DK_ROWS, tile_k = DK_WORDS * (32 / bits), KT = (K + tile_k - 1) / tile_k;
+    if (RB > SMS) return K >= (M <= 16 ? 2560 : 5120);
+    const int per_rb = dec_ctas_per_block(RB, KT, SMS);
+    if (RB > (per_rb == 8 ? 15 : (per_rb == 4 ? 33 : SMS))) return false;
+    const int64_t ctas = RB * per_rb, tiles = (KT + per_rb - 1) / per_rb;
+    if (ctas >= 104 && tiles >= (bits == 8 ? 9 : 4)) return true;
+    if (M > 16 && bits < 8 && ctas >= 64 && tiles >= 5) return true;
+    return per_rb == 8 && K >= 16384;
+}
 
 // Layout preconditions of the persistent decode kernel: at most 32 tokens, power-of-two groups
 // that hold a lane's 16-byte chunk (4 words), rows of packed words and activations that TMA can stride
@@ -981,7 +1006,7 @@ bool decode_path_ok(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K,
     if ((N + DK_ROWS - 1) / DK_ROWS * ((K / vpi + DK_WORDS - 1) / DK_WORDS) > (int64_t)1 << 30) return false;
     if (!aligned_to(q, 16)) return false;
     // (the gated epilogue is only offered where scales and zero points come by TMA)
-    if (!dec_const_tma(scale, zp, K, g) && (!dec_direct_consts(M, N, K) || current_epilogue().act == BW_ACT_SILU_MUL)) return false;
+    if (!dec_const_tma(scale, zp, K, g) && (!dec_direct_consts(M, N, K, bits) || current_epilogue().act == BW_ACT_SILU_MUL)) return false;
     if (!aligned_to(x, 16) || (K * dtype_size(x_dtype)) % 16 != 0) return false;
     return encode_tiled_fn() != nullptr;
 }

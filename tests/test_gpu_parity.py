@@ -551,13 +551,20 @@ def test_persistent_decode_kernel_vs_oracle(case):
         assert_close_rms(as_f32(yb), as_f32(refb), 1e-2, str(case))
 
 
-@pytest.mark.parametrize("bits,g,N,K", [
-    # scales in rows of whole 16-byte units (TMA) or not; ragged last k-tiles and row blocks; clusters, whole row
-    # blocks, shares of several CTAs (N > 148 * 128); just below and above the line for direct scales
-    (4, 128, 384, 4096), (4, 32, 3300, 1312), (4, 128, 1000, 11008), (4, 64, 4000, 1088), (8, 16, 129, 640), (8, 128, 2978, 1408),
-    (8, 128, 2979, 1408), (2, 64, 2048, 2112), (2, 128, 500, 8576), (4, 128, 19200, 1152), (8, 32, 20000, 544),
+@pytest.mark.parametrize("bits,g,N,K,tokens", [
+    # scales in rows of whole 16-byte units: they come by TMA, and every token count runs on the decode kernel
+    (4, 128, 384, 4096, (1, 32)), (8, 16, 129, 640, (1, 32)),
+    # not: loaded directly, for the token counts given; clusters of 8, 4 and 2, whole row blocks, shares through the
+    # scratch (N > 148 * 128), ragged last k-tiles and row blocks
+    (4, 128, 256, 16512, (9, 32)), (2, 64, 256, 16448, (9, 32)), (8, 128, 300, 16512, (9, 32)), (4, 128, 4000, 4480, (9, 32)),
+    (8, 128, 3330, 4480, (9, 32)), (2, 128, 3330, 10368, (9, 32)), (4, 128, 6700, 2176, (9, 32)), (4, 128, 13400, 1152, (9, 32)),
+    (4, 128, 19200, 5248, (9, 32)), (8, 32, 20000, 2592, (9, 16)), (4, 128, 1000, 11008, (17, 32)),
+    # where the cluster split-K kernel is faster: few weights, few CTAs, few tiles, clusters that are not all resident
+    (4, 32, 3300, 1312, None), (4, 64, 4000, 1088, None), (8, 128, 2978, 1408, None), (8, 128, 2979, 1408, None), (2, 64, 2048, 2112, None),
+    (2, 128, 500, 8576, None), (4, 128, 19200, 1152, None), (8, 32, 20000, 544, None), (4, 128, 2048, 8448, None),
+    (4, 128, 4480, 4480, None), (8, 128, 4864, 2176, None),
 ])
-def test_decode_kernel_matches_float64(bits, g, N, K):
+def test_decode_kernel_matches_float64(bits, g, N, K, tokens):
     gen = torch.Generator(device=DEV).manual_seed(N + K)
     q = torch.randint(-2 ** 31, 2 ** 31 - 1, (N, K * bits // 32), generator=gen, device=DEV, dtype=torch.int32)
     s = (torch.rand(N, K // g, generator=gen, device=DEV) * 0.02 + 0.001).half()
@@ -568,8 +575,9 @@ def test_decode_kernel_matches_float64(bits, g, N, K):
         for xdt in (torch.float16, torch.bfloat16) if M != 17 else (torch.float32,):
             x = torch.randn(M, K, generator=gen, device=DEV).to(xdt)
             y = quantized_matmul_cuda(x, q, s, z, b if M % 2 else None, bits, g, out_dtype=torch.float32)
-            if xdt != torch.float32 and ((K // g) % 8 == 0 or (M > 8 and N * K >= 1 << 22)):
-                assert _lib.last_qmatmul_kernel() == "qmm_decode_kernel", (M, xdt)
+            if xdt != torch.float32:
+                decode = tokens is not None and tokens[0] <= M <= tokens[1]
+                assert _lib.last_qmatmul_kernel() == ("qmm_decode_kernel" if decode else "qmm_smallm_kernel"), (M, xdt)
             xh = x.half().double()
             ref = xh @ w.T + (b.double() if M % 2 else 0.0)
             # fp32 sums: a few roundings of partial sums of the order of |x| . |W|
@@ -631,6 +639,9 @@ def test_rtn_batched_call_equals_single_calls_bit_for_bit():
     # cluster split-K streaming kernel, general kernel, tensor-core GEMM (plain and split-K)
     (4, 128, 4, 1024, 4096), (4, 128, 16, 14336, 1024), (4, 128, 3, 20000, 1024), (4, 16, 5, 320, 512),
     (4, 24, 7, 64, 96), (4, 128, 64, 1024, 2048), (4, 128, 300, 512, 1024), (2, 64, 4096, 256, 512),
+    # decode with directly loaded scales: two and four token tiles, every bit width
+    (4, 128, 16, 4000, 4480), (8, 128, 32, 3330, 4480), (2, 64, 17, 256, 16448), (2, 128, 9, 3330, 10368), (4, 128, 24, 6700, 2176),
+    (8, 128, 12, 300, 16512),
 ], ids=lambda c: "b%d_g%d_M%d_N%d_K%d" % c)
 def test_fused_relu_and_residual_equal_the_separate_ops(case):
     # bw_qmatmul_fused: relu(linear) + residual inside the kernel's output stage must give the
@@ -642,6 +653,7 @@ def test_fused_relu_and_residual_equal_the_separate_ops(case):
     dev = [t.to(DEV) for t in (q, s_h, z_h, b_h)]
     plain = quantized_matmul_cuda(x, *dev, bits, g)
     kern = _lib.last_qmatmul_kernel()
+    assert kern == "qmm_decode_kernel" or M > 32 or g < 32
     fused = quantized_matmul_cuda(x, *dev, bits, g, activation="relu", residual=res)
     assert _lib.last_qmatmul_kernel() == kern
     assert torch.equal(fused, torch.relu(plain) + res), (case, kern)
