@@ -8,7 +8,7 @@
 namespace bw {
 
 static thread_local char g_cuda_error[256] = "";
-static thread_local const char *g_last_kernel = "";
+static thread_local const char *g_last_kernel = "", *g_last_launch = "";
 static thread_local Epilogue g_epilogue = {BW_ACT_NONE, nullptr};
 Epilogue current_epilogue() { return g_epilogue; }
 
@@ -18,7 +18,8 @@ int record_cuda_error(cudaError_t e, const char *where) {
     (void)cudaGetLastError();  // clear the sticky-free error state for the next call
     return BW_ERR_CUDA;
 }
-void set_last_kernel(const char *name) { g_last_kernel = name; }
+void set_last_kernel(const char *name) { g_last_kernel = g_last_launch = name; }
+void note_launch(const char *name) { g_last_launch = name; }
 
 // implemented in the kernel translation units
 int rtn_quantize_pack(const void *w, int w_dtype, int64_t N, int64_t K, int bits, int g, int32_t *q,
@@ -550,6 +551,7 @@ int bw_device_status(void) {
 }
 int bw_version(void) { return 100; }
 const char *bw_last_qmatmul_kernel(void) { return g_last_kernel; }
+const char *bw_last_kernel(void) { return g_last_launch; }
 
 #ifdef BW_TUNING
 // Tuning build only (-DBW_TUNING): process-wide, unsynchronised switches for kernel experiments.

@@ -11,7 +11,8 @@ namespace bw {
 
 // Records a failed CUDA runtime call for bw_last_cuda_error(); returns BW_ERR_CUDA.
 int record_cuda_error(cudaError_t e, const char *where);
-void set_last_kernel(const char *name);
+void set_last_kernel(const char *name);      // of a bw_qmatmul call, once its route is known
+void note_launch(const char *name);          // any kernel that was launched
 
 #define BW_CUDA_TRY(expr)                                              \
     do {                                                               \
@@ -21,7 +22,9 @@ void set_last_kernel(const char *name);
 
 inline int check_launch(const char *where) {
     cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? BW_OK : record_cuda_error(e, where);
+    if (e != cudaSuccess) return record_cuda_error(e, where);
+    note_launch(where);
+    return BW_OK;
 }
 
 inline bool aligned_to(const void *p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }

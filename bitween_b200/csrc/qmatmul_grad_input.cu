@@ -725,6 +725,7 @@ int launch_umma(const void *go, int64_t M, int64_t N, int64_t K, const int32_t *
         cfg.numAttrs = 1;
     }
     BW_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, xm, wm, sm, zm, om, p));
+    note_launch("grad_input_umma_kernel");
     return BW_OK;
 }
 

@@ -366,10 +366,13 @@ rtn_quantize_pack_kernel(const T *__restrict__ w, int64_t total_chunks, int cpg_
 // Codes on the fp32 path: the reference's code is rint(RN(RN(v/s) + zp)).  t = RN(v*r + zp) with
 // r = RN(1/s) differs from the value inside rint() by at most 2.5 * 2^(BITS-24) while |v/s| <=
 // 2^BITS (r: 2^BITS * 2^-24; three roundings of half an ulp of 2^BITS), so unless t lies within
-// EPS = 2^(BITS-22) of a tie both round to the same integer -- and that integer needs no clamp when the
-// group's range contains zero (the value then lies in [-1/2, Qmax + 1/2]).  A thread with a weight in
-// that margin (1 in 8000 weights at 8 bits, 1 in 130000 at 4) and warps with a group on one side of
-// zero take the exact quotient (div_by_recip) and the clamps instead.
+// EPS = 4 * 2^(BITS-24) of a tie both round to the same integer.  That integer needs no clamp when the
+// group's range contains zero, and EPS may not be smaller for that: (max - min) / s exceeds Qmax by up to
+// Qmax * 2^-23 (roundings of max - min and of s), the quotient under zp and the last rounding of t add theirs,
+// so t lies in [-1/2 - 3.5 * 2^(BITS-24), Qmax + 1/2 + 3.5 * 2^(BITS-24)] -- past the tie at Qmax + 1/2, where
+// it would round to Qmax + 1, but within the margin.  A thread with a weight in the margin (1 in 8000
+// weights at 8 bits, 1 in 130000 at 4) and warps with a group on one side of zero take the exact quotient
+// (div_by_recip) and the clamps instead.
 //
 // Measured against the 16-byte form: 4096 x 4096 fp32 -> W8 g32 16.9 us (5.2 TB/s) instead of 24.8; the seven
 // linears of a Llama-3-8B block, bf16 -> W4 g128 in one batch, 173 us (3.2 TB/s) instead of 211 -- there the
@@ -774,11 +777,11 @@ thread_local bool t_rtn_stream = false;
 struct RtnBatchCall { const RtnBatchEntry *table; int njobs; long long blocks; bool wide; };
 thread_local RtnBatchCall t_rtn_batch = {nullptr, 0, 0, false};
 
-// The wide form: groups of whole 64-byte units, at most a warp of them, weights aligned to its 32-byte loads
-// and packed words to its 16-byte stores.  (Smaller groups share a unit: 16-byte chunks.)
+// The wide form among the calls that the 16-byte form could take (groups of a power of two of 16-byte chunks, at
+// most 32 of them): groups of whole 64-byte units, that is 1 to 8 lanes, weights aligned to its 32-byte loads and
+// packed words to its 16-byte stores.  (Smaller groups share a unit; larger ones run on the general kernel.)
 inline bool rtn_wide_ok(const void *w, const void *q, size_t elem, int g) {
-    const size_t bytes = (size_t)g * elem, lanes = bytes / 64;
-    return bytes % 64 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && aligned_to(w, 32) && aligned_to(q, 16);
+    return (size_t)g * elem % 64 == 0 && aligned_to(w, 32) && aligned_to(q, 16);
 }
 
 int64_t gcd64(int64_t a, int64_t b) { while (b) { int64_t t = a % b; a = b; b = t; } return a; }

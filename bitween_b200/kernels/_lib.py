@@ -111,6 +111,8 @@ def _declare(L):
     L.bw_last_cuda_error.restype = ctypes.c_char_p
     L.bw_last_qmatmul_kernel.argtypes = []
     L.bw_last_qmatmul_kernel.restype = ctypes.c_char_p
+    L.bw_last_kernel.argtypes = []
+    L.bw_last_kernel.restype = ctypes.c_char_p
     L.bw_version.argtypes = []
     L.bw_version.restype = i32
     L.bw_device_status.argtypes = []
@@ -211,3 +213,7 @@ def current_workspace(device, raw_stream):
 
 def last_qmatmul_kernel():
     return lib().bw_last_qmatmul_kernel().decode()
+
+
+def last_kernel():
+    return lib().bw_last_kernel().decode()

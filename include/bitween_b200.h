@@ -386,6 +386,9 @@ BW_API int bw_version(void);
 BW_API long long bw_selftest_division(unsigned long long n, unsigned long long seed);
 /* Name of the kernel the last bw_qmatmul call of this thread dispatched to (diagnostics). */
 BW_API const char *bw_last_qmatmul_kernel(void);
+/* Name of the kernel that the last call of any kind on this thread ran (quantization, dequantization
+ * and the backward pass included): which of several forms a layout took. */
+BW_API const char *bw_last_kernel(void);
 
 #ifdef __cplusplus
 }

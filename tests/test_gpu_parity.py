@@ -196,11 +196,11 @@ def _awkward_weights(N, K, g, bits, dt, seed):
 @pytest.mark.parametrize("bits", [2, 4, 8])
 @pytest.mark.parametrize("dt", [torch.float32, torch.float16, torch.bfloat16], ids=str)
 def test_rtn_wide_units_match_oracle_on_awkward_groups(bits, dt):
-    # 64-byte units (one to 32 lanes a group), a last block that is not whole, and the same weights 16 bytes off
-    # a 32-byte boundary (16-byte chunks): one result, the oracle's, bit for bit
+    # 64-byte units (one to 8 lanes a group), a last block that is not whole, and the same weights 16 bytes off
+    # a 32-byte boundary (16-byte chunks): one result, the oracle's, bit for bit.  (Groups beyond 512 bytes, and below 64:
+    # the other two forms.)
     for N, K, g in ((7, 512, 32), (3, 1024, 64), (65, 1280, 128), (33, 1024, 512), (3, 2048, 1024), (9, 96, 16)):
-        if g * (4 if dt == torch.float32 else 2) // 64 > 32:
-            continue
+        nbytes = g * (4 if dt == torch.float32 else 2)
         w = _awkward_weights(N, K, g, bits, dt, 17 * bits + g)
         qo, so, zo = oracle.quantize_rtn(to_np(w), ORACLE_DT[dt], bits, g)
         pad = 16 // w.element_size()
@@ -208,6 +208,9 @@ def test_rtn_wide_units_match_oracle_on_awkward_groups(bits, dt):
         assert shifted.data_ptr() % 32 == 16
         for dev in (w.to(DEV), shifted):
             q, s, z, _ = quantize_rtn(dev, bits=bits, group_size=g)
+            kernel = "rtn_quantize_pack_general_kernel" if nbytes > 512 else \
+                "rtn_quantize_pack_kernel" if dev is shifted or nbytes < 64 else "rtn_quantize_pack_wide_kernel"
+            assert _lib.last_kernel() == kernel, (N, K, g)
             assert _bits_equal(q, qo) and _bits_equal(z, zo), (N, K, g)
             ns = torch.isnan(s.cpu())
             assert torch.equal(ns, torch.isnan(from_bits(so, dt) if dt != torch.float32 else torch.from_numpy(so)))
@@ -220,8 +223,10 @@ def test_rtn_wide_units_match_oracle_on_awkward_groups(bits, dt):
 
 @pytest.mark.parametrize("bits", [2, 4, 8])
 def test_dequantize_words_kernel_matches_oracle(bits):
-    # power-of-two words per group, sizes around the four-words-a-thread blocks, aligned and misaligned outputs
+    # power-of-two words per group, sizes around the four-words-a-thread blocks; outputs on a 32-byte boundary, and off
+    # it by one element up to 16 bytes through the C call (one word a thread, as for other groups)
     vpi = 32 // bits
+    L = _lib.lib()
     for N, K, g in ((1, vpi, vpi), (3, 1024, 128), (129, 32 * vpi, 2 * vpi), (1, 4097 * vpi, vpi), (5, 96 * vpi, 3 * vpi)):
         gen = torch.Generator().manual_seed(N + K)
         q = torch.randint(-2 ** 31, 2 ** 31 - 1, (N, K // vpi), generator=gen, dtype=torch.int32)
@@ -229,8 +234,18 @@ def test_dequantize_words_kernel_matches_oracle(bits):
         z = torch.randint(0, 2 ** bits, (N, K // g), generator=gen, dtype=torch.int32)
         ref = oracle.dequantize_rtn(to_np(q), to_np(s), to_np(z), g, bits)
         for out_dtype in (torch.float32, torch.float16, torch.bfloat16):
-            got = dequantize_rtn(q.to(DEV), s.to(DEV), z.to(DEV), g, bits=bits, out_dtype=out_dtype)
-            assert torch.equal(got.cpu(), torch.from_numpy(ref).to(out_dtype)), (N, K, g, out_dtype)
+            dev, want = [t.to(DEV) for t in (q, s, z)], torch.from_numpy(ref).to(out_dtype)
+            got = dequantize_rtn(*dev, g, bits=bits, out_dtype=out_dtype)
+            assert _lib.last_kernel() == ("dequantize_kernel" if g == 3 * vpi else "dequantize_words_kernel")
+            assert torch.equal(got.cpu(), want), (N, K, g, out_dtype)
+            for off in {got.element_size(), 4, 8, 16}:
+                buf = torch.zeros(N * K * got.element_size() + 64, dtype=torch.uint8, device=DEV)
+                rc = L.bw_dequantize(dev[0].data_ptr(), dev[1].data_ptr(), _lib.F32, dev[2].data_ptr(), _lib.I32, N, K, bits, g,
+                                     buf.data_ptr() + off, _lib.dtype_code(out_dtype), _lib.raw_stream(buf.device))
+                assert rc == 0 and _lib.last_kernel() == "dequantize_kernel"
+                out = buf[off:off + N * K * got.element_size()].clone().view(out_dtype).view(N, K)
+                assert torch.equal(out.cpu(), want), (N, K, g, out_dtype, off)
+                assert not bool(buf[:off].any()) and not bool(buf[off + N * K * got.element_size():].any())
 
 
 def test_rtn_error_bound_full_size_layer():
@@ -634,6 +649,36 @@ def test_rtn_batched_call_equals_single_calls_bit_for_bit():
     assert _lib.lib().bw_device_status() == 0
 
 
+def test_rtn_batched_call_takes_every_form():
+    # one launch of 16-byte chunks (groups below 64 bytes, one matrix off a 32-byte boundary), one of 64-byte units beside
+    # an empty matrix: the single calls' results
+    from bitween_b200.functional import quantize_rtn_many_to_module_buffers
+    gen = torch.Generator(device=DEV).manual_seed(22)
+    for dt, bits, g, off, kernel in ((torch.bfloat16, 4, 16, 0, "rtn_quantize_pack_batch_kernel"),
+                                     (torch.float16, 2, 16, 0, "rtn_quantize_pack_batch_kernel"),
+                                     (torch.float32, 8, 8, 0, "rtn_quantize_pack_batch_kernel"),
+                                     (torch.bfloat16, 4, 128, 16, "rtn_quantize_pack_batch_kernel"),
+                                     (torch.float32, 8, 32, 16, "rtn_quantize_pack_batch_kernel"),
+                                     (torch.bfloat16, 4, 128, 0, "rtn_quantize_pack_wide_batch_kernel"),
+                                     (torch.float32, 8, 32, 0, "rtn_quantize_pack_wide_batch_kernel"),
+                                     (torch.float16, 2, 256, 0, "rtn_quantize_pack_wide_batch_kernel")):
+        ws = []
+        for n, k in ((130, 768), (0, 512), (1, 256), (513, 1280)):
+            flat = torch.empty(n * k + 64, dtype=dt, device=DEV)
+            pad = off // flat.element_size() if n == 513 else 0
+            ws.append(flat[pad:pad + n * k].view(n, k).copy_(torch.randn(n, k, device=DEV, generator=gen) * 0.02))
+        assert ws[3].data_ptr() % 32 == off
+        many = quantize_rtn_many_to_module_buffers(ws, bits, g)
+        assert _lib.last_kernel() == kernel, (dt, bits, g)
+        for w, (q, s, z) in zip(ws, many):
+            q1, s1, z1 = quantize_rtn_to_module_buffers(w, bits, g)
+            assert torch.equal(q, q1) and torch.equal(s, s1) and torch.equal(z, z1), (dt, bits, g, tuple(w.shape))
+        qo, so, zo = oracle.quantize_rtn(to_np(ws[3].float()), oracle.F32, bits, g)
+        assert _bits_equal(many[3][0], qo) and _bits_equal(many[3][1], oracle.f16_bits(so))
+        assert _bits_equal(many[3][2], oracle.f16_bits(zo.astype(np.float32)))
+    assert _lib.lib().bw_device_status() == 0
+
+
 @pytest.mark.parametrize("case", [
     # bits, g, M, N, K -- one case per kernel: decode (clusters, whole row blocks, stream-K),
     # cluster split-K streaming kernel, general kernel, tensor-core GEMM (plain and split-K)
@@ -670,19 +715,35 @@ def test_fused_relu_and_residual_equal_the_separate_ops(case):
     assert _lib.lib().bw_device_status() == 0
 
 
-@pytest.mark.parametrize("bits,g,gdt,shape", [
-    (4, 128, torch.float16, (300, 200, 384)), (4, 64, torch.bfloat16, (129, 48, 192)),
-    (8, 32, torch.float16, (16, 130, 96)), (2, 64, torch.bfloat16, (257, 64, 1024)), (4, 24, torch.float16, (33, 18, 96)),
+@pytest.mark.parametrize("bits,g,gdt,shape,kernel", [
+    (4, 128, torch.float16, (300, 200, 384), "grad_input_umma_kernel"), (4, 64, torch.bfloat16, (129, 48, 192), "grad_input_umma_kernel"),
+    (8, 32, torch.float16, (16, 130, 96), "grad_input_tc_kernel"), (2, 64, torch.bfloat16, (257, 64, 1024), "grad_input_umma_kernel"),
+    (4, 24, torch.float16, (33, 18, 96), "grad_input_tc_kernel"),
+    # rows of gradients that TMA cannot stride over (N not a multiple of 8): every bit width, several token blocks and
+    # column blocks
+    (2, 64, torch.float16, (300, 202, 384), "grad_input_tc_kernel"), (2, 128, torch.bfloat16, (129, 66, 640), "grad_input_tc_kernel"),
+    (4, 128, torch.bfloat16, (257, 130, 384), "grad_input_tc_kernel"), (4, 32, torch.float16, (129, 50, 192), "grad_input_tc_kernel"),
+    (8, 32, torch.bfloat16, (130, 70, 320), "grad_input_tc_kernel"), (8, 128, torch.float16, (257, 34, 256), "grad_input_tc_kernel"),
+    (4, 128, torch.float16, (20, 33, 256), "grad_input_kernel"),
 ], ids=lambda v: str(v).replace(" ", ""))
-def test_grad_input_tensor_core_kernel_vs_oracle(bits, g, gdt, shape):
-    # 16-bit gradients run on mma.sync tiles of 128 tokens x 64 k over steps of 16 weight rows:
-    # ragged M, N and K tails, every bit width, groups that split a packed word (g = 24)
+def test_grad_input_tensor_core_kernel_vs_oracle(bits, g, gdt, shape, kernel):
+    # 16-bit gradients run on the tcgen05 kernel where TMA can stride over their rows, else on mma.sync tiles of 128
+    # tokens x 64 k over steps of 16 weight rows: ragged M, N and K tails, every bit width, groups that split a packed
+    # word (g = 24)
     M, N, K = shape
     q, s_h, z_h, _ = _make_layer(950 + bits + M, N, K, bits, g, False)
     go = torch.from_numpy(synth.normal(951, (M, N), 1.0)).to(gdt)
     ref = from_bits(oracle.qlinear_grad_input(to_np(go), ORACLE_DT[gdt], to_np(q), to_np(s_h), to_np(z_h), bits, g), gdt)
     gi = quantized_matmul_grad_input(go.to(DEV), q.to(DEV), s_h.to(DEV), z_h.to(DEV), bits, g)
-    assert gi.dtype == gdt and tuple(gi.shape) == (M, K)
+    assert gi.dtype == gdt and tuple(gi.shape) == (M, K) and _lib.last_kernel() == kernel
+    if kernel == "grad_input_umma_kernel":
+        # the same gradients 8 bytes off a 16-byte boundary: not for TMA
+        off = torch.empty(M * N + 4, dtype=gdt, device=DEV)[4:].view(M, N).copy_(go)
+        gi_off = quantized_matmul_grad_input(off, q.to(DEV), s_h.to(DEV), z_h.to(DEV), bits, g)
+        assert _lib.last_kernel() == "grad_input_tc_kernel"
+        # (sums in another order; two results may round to neighbouring 16-bit numbers)
+        ulp = 2.0 ** (-7 if gdt == torch.bfloat16 else -10) * np.abs(as_f32(gi))
+        assert (np.abs(as_f32(gi_off) - as_f32(gi)) <= 1e-5 * rms(as_f32(gi)) * N + ulp).all()
     if gdt == torch.bfloat16:
         # one bf16 ulp of the value on top of the bar: the final rounding alone moves a value by
         # up to 2^-8 |y|, more than 1e-2 * RMS for |y| > 2.6 RMS, whenever the fp32 sums differ
@@ -703,9 +764,10 @@ def test_grad_input_tensor_core_kernel_vs_oracle(bits, g, gdt, shape):
                                         (4, 64, torch.bfloat16), (8, 16, torch.bfloat16), (8, 32, torch.float16), (8, 256, torch.float16)])
 def test_grad_input_tiles_match_float64(bits, g, gdt):
     # token tiles of 16 .. 256 and their remainders, a last column tile and a last stage of rows that are not
-    # whole, rows split over a cluster, several tiles per CTA, scales that TMA can fetch (groups a multiple of 8) or not
+    # whole, rows split over a cluster (a CTA of it without rows: 33 stages over 8), several tiles per CTA, scales that TMA
+    # can fetch (groups a multiple of 8) or not
     for M, N, K in ((1, 8, 256), (16, 64, 512), (17, 72, 768), (33, 1000, 512), (64, 4096, 1024), (65, 136, 1280), (129, 520, 2048),
-                    (256, 64, 256 + (128 if g <= 128 else 256)), (257, 1032, 1024), (1030, 256, 8192 + 256)):
+                    (256, 64, 256 + (128 if g <= 128 else 256)), (257, 1032, 1024), (1030, 256, 8192 + 256), (40, 2112, 512)):
         gen = torch.Generator(device=DEV).manual_seed(M + bits)
         q = torch.randint(-2 ** 31, 2 ** 31 - 1, (N, K * bits // 32), generator=gen, device=DEV, dtype=torch.int32)
         s = (torch.rand(N, K // g, generator=gen, device=DEV) * 0.02 + 0.001).half()
@@ -716,6 +778,7 @@ def test_grad_input_tiles_match_float64(bits, g, gdt):
         w = dequantize_rtn(q, s, z, g, bits=bits).to(gdt).double()
         ref = go.double() @ w
         gi = quantized_matmul_grad_input(go, q, s, z, bits, g).double()
+        assert _lib.last_kernel() == "grad_input_umma_kernel"
         # one rounding of the result, and fp32 sums that the tensor core truncates once per 16 terms, each
         # partial sum of the order of |go| . |W|
         slack = 2.0 ** (-8 if gdt == torch.bfloat16 else -11) * ref.abs() + N / 16 * 2.0 ** -23 * (go.double().abs() @ w.abs()) + 1e-7
