@@ -647,6 +647,18 @@ bool encode_2d(CUtensorMap *map, CUtensorMapDataType dt, const void *base, int64
                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Products that the mma.sync kernel does faster: one or two steps of weight rows and at most about two of its blocks an
+// SM.  The tcgen05 kernel's fixed part (rings, tensor memory, 24 warps; 4.5 us, 7 us with a tile of 256 tokens) is then
+// the whole call; at 8 bits a step there costs twice as much.  us there / here, W4 g128: N 64, K 1024: 4.1 / 5.2 at 64
+// tokens, 5.0 / 7.5 at 1024; N 96, K 1024: 6.0 / 5.3 at 64, 7.2 / 7.7 at 1024; N 128: 6.7 / 5.4 and 8.3 / 7.6; N 64,
+// K 4096: 11.7 / 7.8 at 1024 tokens.  W8 g32: N 64, K 4096: 6.0 / 7.6 at 256 tokens, 9.0 / 7.6 at 512.
+bool grad_small(int64_t M, int64_t N, int64_t K, int bits) {
+    if (M > (1 << 20) || K > (1 << 20)) return false;
+    const int64_t blocks = (M + GI_BM - 1) / GI_BM * ((K + GI_BK - 1) / GI_BK);
+    const int64_t room = (M > 128 ? 16384 : 8192) / (bits == 8 ? 2 : 1);
+    return N <= (M > 128 && bits < 8 ? 120 : 64) && blocks <= 256 && N * blocks <= room;
+}
+
 // What the tcgen05 kernel can take: 16-bit gradients in rows that TMA can stride over (whole 16-byte units,
 // 16-byte aligned), power-of-two groups of at least 16 codes that hold whole words, whole 16-byte vectors
 // of packed words per row, at least one full tile of columns.  The rest runs on the kernels above.
@@ -744,7 +756,7 @@ int launch(const void *go, int64_t M, int64_t N, int64_t K, const int32_t *q, co
 template <int BITS>
 int launch_dt(const void *go, int dt, int64_t M, int64_t N, int64_t K, const int32_t *q,
               const __half *scale, const __half *zp, void *gi, int g, cudaStream_t st) {
-    if (grad_umma_ok(go, gi, dt, M, N, K, q, BITS, g)) {
+    if (grad_umma_ok(go, gi, dt, M, N, K, q, BITS, g) && !grad_small(M, N, K, BITS)) {
         const int rc = dt == BW_F16 ? launch_umma<BITS, __half>(go, M, N, K, q, scale, zp, gi, g, st)
                                     : launch_umma<BITS, __nv_bfloat16>(go, M, N, K, q, scale, zp, gi, g, st);
         if (rc != BW_ERR_UNSUPPORTED) return rc;

@@ -716,9 +716,11 @@ def test_fused_relu_and_residual_equal_the_separate_ops(case):
 
 
 @pytest.mark.parametrize("bits,g,gdt,shape,kernel", [
-    (4, 128, torch.float16, (300, 200, 384), "grad_input_umma_kernel"), (4, 64, torch.bfloat16, (129, 48, 192), "grad_input_umma_kernel"),
-    (8, 32, torch.float16, (16, 130, 96), "grad_input_tc_kernel"), (2, 64, torch.bfloat16, (257, 64, 1024), "grad_input_umma_kernel"),
-    (4, 24, torch.float16, (33, 18, 96), "grad_input_tc_kernel"),
+    (4, 128, torch.float16, (300, 200, 384), "grad_input_umma_kernel"), (4, 64, torch.bfloat16, (129, 152, 192), "grad_input_umma_kernel"),
+    (8, 32, torch.float16, (16, 136, 128), "grad_input_umma_kernel"), (2, 64, torch.bfloat16, (257, 128, 1024), "grad_input_umma_kernel"),
+    # few weight rows
+    (4, 64, torch.bfloat16, (129, 48, 192), "grad_input_tc_kernel"), (2, 64, torch.bfloat16, (257, 64, 1024), "grad_input_tc_kernel"),
+    (8, 32, torch.float16, (16, 130, 96), "grad_input_tc_kernel"), (4, 24, torch.float16, (33, 18, 96), "grad_input_tc_kernel"),
     # rows of gradients that TMA cannot stride over (N not a multiple of 8): every bit width, several token blocks and
     # column blocks
     (2, 64, torch.float16, (300, 202, 384), "grad_input_tc_kernel"), (2, 128, torch.bfloat16, (129, 66, 640), "grad_input_tc_kernel"),
@@ -766,8 +768,10 @@ def test_grad_input_tiles_match_float64(bits, g, gdt):
     # token tiles of 16 .. 256 and their remainders, a last column tile and a last stage of rows that are not
     # whole, rows split over a cluster (a CTA of it without rows: 33 stages over 8), several tiles per CTA, scales that TMA
     # can fetch (groups a multiple of 8) or not
-    for M, N, K in ((1, 8, 256), (16, 64, 512), (17, 72, 768), (33, 1000, 512), (64, 4096, 1024), (65, 136, 1280), (129, 520, 2048),
-                    (256, 64, 256 + (128 if g <= 128 else 256)), (257, 1032, 1024), (1030, 256, 8192 + 256), (40, 2112, 512)):
+    few = ((1, 8, 256), (16, 64, 512), (256, 64, 256 + (128 if g <= 128 else 256)), (128, 64, 4096))      # mma.sync
+    few += ((129, 120, 4096),) if bits < 8 else ((129, 64, 4096),)
+    for M, N, K in few + ((129, 128, 4096) if bits < 8 else (129, 72, 4096), (1, 72, 256), (16, 64, 8448), (17, 72, 768), (33, 1000, 512), (64, 4096, 1024), (65, 136, 1280), (129, 520, 2048),
+                          (129, 128, 512), (2100, 8, 1024), (257, 1032, 1024), (1030, 256, 8192 + 256), (40, 2112, 512)):
         gen = torch.Generator(device=DEV).manual_seed(M + bits)
         q = torch.randint(-2 ** 31, 2 ** 31 - 1, (N, K * bits // 32), generator=gen, device=DEV, dtype=torch.int32)
         s = (torch.rand(N, K // g, generator=gen, device=DEV) * 0.02 + 0.001).half()
@@ -778,7 +782,7 @@ def test_grad_input_tiles_match_float64(bits, g, gdt):
         w = dequantize_rtn(q, s, z, g, bits=bits).to(gdt).double()
         ref = go.double() @ w
         gi = quantized_matmul_grad_input(go, q, s, z, bits, g).double()
-        assert _lib.last_kernel() == "grad_input_umma_kernel"
+        assert _lib.last_kernel() == ("grad_input_tc_kernel" if (M, N, K) in few else "grad_input_umma_kernel"), (M, N, K)
         # one rounding of the result, and fp32 sums that the tensor core truncates once per 16 terms, each
         # partial sum of the order of |go| . |W|
         slack = 2.0 ** (-8 if gdt == torch.bfloat16 else -11) * ref.abs() + N / 16 * 2.0 ** -23 * (go.double().abs() @ w.abs()) + 1e-7
