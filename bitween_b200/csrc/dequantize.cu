@@ -121,7 +121,10 @@ int launch4(const int32_t *q, const ST *s, const ZT *z, int64_t N, int64_t K, in
     const int64_t total = N * wpr;
     if (total == 0) return BW_OK;
     const int wpg = g / VPI;
-    if (g % VPI == 0 && (wpg & (wpg - 1)) == 0 && aligned_to(out, 32) && (total + 1023) / 1024 <= 0x7fffffff) {
+    // (2 bits, fewer blocks of four words a thread than half the SMs: 16 outputs a word leave too few threads to write
+    // them.  512 x 512 -> fp32 2.8 us there, 2.4 at a word a thread; 1024 x 1024 2.9 and 3.2.)
+    const bool few = BITS == 2 && total > 1024 && total < (1 << 16);
+    if (!few && g % VPI == 0 && (wpg & (wpg - 1)) == 0 && aligned_to(out, 32) && (total + 1023) / 1024 <= 0x7fffffff) {
         int sh = 0;
         while ((1 << sh) < wpg) ++sh;
         dequantize_words_kernel<BITS, ST, ZT, OutT><<<(unsigned)((total + 1023) / 1024), 256, 0, st>>>(q, s, z, total, sh, out);

@@ -227,7 +227,9 @@ def test_dequantize_words_kernel_matches_oracle(bits):
     # it by one element up to 16 bytes through the C call (one word a thread, as for other groups)
     vpi = 32 // bits
     L = _lib.lib()
-    for N, K, g in ((1, vpi, vpi), (3, 1024, 128), (129, 32 * vpi, 2 * vpi), (1, 4097 * vpi, vpi), (5, 96 * vpi, 3 * vpi)):
+    for N, K, g in ((1, vpi, vpi), (3, 1024, 128), (129, 32 * vpi, 2 * vpi), (1, 4097 * vpi, vpi), (5, 96 * vpi, 3 * vpi),
+                    (2048, 32 * vpi, 2 * vpi), (1, 65537 * vpi, vpi)):
+        few = bits == 2 and 1024 < N * K // vpi < 65536
         gen = torch.Generator().manual_seed(N + K)
         q = torch.randint(-2 ** 31, 2 ** 31 - 1, (N, K // vpi), generator=gen, dtype=torch.int32)
         s = torch.rand(N, K // g, generator=gen) * 0.02
@@ -236,7 +238,7 @@ def test_dequantize_words_kernel_matches_oracle(bits):
         for out_dtype in (torch.float32, torch.float16, torch.bfloat16):
             dev, want = [t.to(DEV) for t in (q, s, z)], torch.from_numpy(ref).to(out_dtype)
             got = dequantize_rtn(*dev, g, bits=bits, out_dtype=out_dtype)
-            assert _lib.last_kernel() == ("dequantize_kernel" if g == 3 * vpi else "dequantize_words_kernel")
+            assert _lib.last_kernel() == ("dequantize_kernel" if few or g == 3 * vpi else "dequantize_words_kernel")
             assert torch.equal(got.cpu(), want), (N, K, g, out_dtype)
             for off in {got.element_size(), 4, 8, 16}:
                 buf = torch.zeros(N * K * got.element_size() + 64, dtype=torch.uint8, device=DEV)
