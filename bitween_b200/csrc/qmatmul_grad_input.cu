@@ -618,13 +618,10 @@ grad_input_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_c
         }
         cluster.sync();                                     // shared memory stays until every peer has read it
     }
+    linger_after_abort(abort_flag);
     tc_fence_before();
     __syncthreads();
     if (warp == 3) tmem_dealloc(tmem_base, tmem_cols);
-    if (*abort_flag) {
-        // copies may still be in flight into this CTA's shared memory
-        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
-    }
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,

@@ -46,6 +46,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, volati
     }
     return true;
 }
+// Before tensor and shared memory are given back: where a wait ran out, copies into this CTA's shared memory and MMAs
+// into its tensor memory may still be in flight (microseconds; this waits about 2 ms).
+__device__ __forceinline__ void linger_after_abort(volatile int *abort_flag) {
+    if (*abort_flag)
+        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+}
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
