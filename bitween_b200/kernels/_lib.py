@@ -161,9 +161,13 @@ def stream_ptr(device):
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
 
 
+# (not public: where a torch build has no such function, the public way, 1 us a call slower, is used)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def raw_stream(device):
     """The current stream of `device` as an integer handle."""
-    return torch._C._cuda_getCurrentRawStream(device.index)
+    return _raw_stream(device.index) if _raw_stream else torch.cuda.current_stream(device).cuda_stream
 
 
 _NO_GUARD = contextlib.nullcontext()

@@ -277,3 +277,13 @@ def test_out_dtype_is_found_wherever_a_subclass_keeps_it(monkeypatch):
             layer.out_dtype = torch.bfloat16
             layer(x)
             assert seen.pop() == (torch.bfloat16,)
+
+
+def test_stream_handle_without_the_private_torch_function(monkeypatch):
+    from types import SimpleNamespace
+    from bitween_b200.kernels import _lib
+    monkeypatch.setattr(_lib, "_raw_stream", None)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device: SimpleNamespace(cuda_stream=40 + device.index))
+    assert _lib.raw_stream(torch.device("cuda", 2)) == 42
+    monkeypatch.setattr(_lib, "_raw_stream", lambda index: index)
+    assert _lib.raw_stream(torch.device("cuda", 3)) == 3
