@@ -618,7 +618,6 @@ grad_input_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_c
         }
         cluster.sync();                                     // shared memory stays until every peer has read it
     }
-    linger_after_abort(abort_flag);
     tc_fence_before();
     __syncthreads();
     if (warp == 3) tmem_dealloc(tmem_base, tmem_cols);

@@ -529,7 +529,6 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
     }
     // the staging tiles must outlive the bulk stores that read them
     if (TMAST) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-    linger_after_abort(abort_flag);
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem_base, tmem_cols);

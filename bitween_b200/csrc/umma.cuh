@@ -32,7 +32,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, unsigned parity) {
     return ok != 0;
 }
 // Bounded wait.  Returns false (and records the error) when the limit is hit or another
-// thread of the CTA has already given up.
+// thread of the CTA has already given up.  The thread that hits the limit stays a few milliseconds: the CTA gives
+// nothing back before it has reached the closing barrier, and copies into its shared memory and MMAs into its tensor
+// memory may still be in flight (microseconds).  (A look at the flag behind that barrier instead cost every launch of
+// a 48-token layer 0.4 us.)
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, volatile int *abort_flag, int code, int *status) {
     unsigned tries = 0;
     while (!mbar_try_wait(bar, parity)) {
@@ -41,16 +44,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, volati
         if (++tries > UMMA_WAIT_LIMIT) {
             *abort_flag = code;
             atomicExch(status, code);
+            for (int i = 0; i < 4; ++i) __nanosleep(1000000);
             return false;
         }
     }
     return true;
-}
-// Before tensor and shared memory are given back: where a wait ran out, copies into this CTA's shared memory and MMAs
-// into its tensor memory may still be in flight (microseconds; this waits about 2 ms).
-__device__ __forceinline__ void linger_after_abort(volatile int *abort_flag) {
-    if (*abort_flag)
-        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
 }
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
