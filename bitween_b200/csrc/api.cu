@@ -49,6 +49,7 @@ int qmatmul_tc(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, cons
 bool decode_path_ok(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, const int32_t *q,
                     const void *scale, const void *zp, int bits, int g);
 size_t decode_workspace_bytes(int64_t M, int64_t N, int64_t K, int bits);
+bool decode_shares_blocks(int64_t N);
 int decode_device_status();
 void set_decode_tuning(int enabled, int smem_kb, int max_ctas, int pdl);
 int qmatmul_decode(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, const int32_t *q,
@@ -169,6 +170,7 @@ size_t bw_qmatmul_workspace_bytes(int64_t M, int64_t N, int64_t K, int bits, int
 }
 
 size_t bw_qmatmul_workspace_bytes_for(int64_t M, int64_t N, int64_t K, int bits, int group_size, int x_dtype, int x_align) {
+    if (M <= 32 && !decode_shares_blocks(N)) return cluster_path_workspace_bytes(M, K, bits);
     const size_t all = bw_qmatmul_workspace_bytes(M, N, K, bits, group_size);
     if (M <= TC_MIN_TOKENS || x_dtype != BW_F16 || x_align < 16) return all;
     // more than 32 tokens of aligned fp16: the GEMM reads them in place; only layouts the GEMM
@@ -218,7 +220,7 @@ static int qmatmul_dispatch(const void *x, int x_dtype, int64_t M, int64_t N, in
     if (!smallm_fast_path_ok(x, x_dtype, K, qweight, bits, group_size))
         return qmatmul_smallm(x, x_dtype, M, N, K, qweight, s, z, b, out, out_dtype, bits, group_size, nullptr, st);
     if (persistent_decode && M <= 32 && decode_path_ok(x, x_dtype, M, N, K, qweight, scale, zero_point, bits, group_size)) {
-        if (!workspace || workspace_bytes < bw_qmatmul_workspace_bytes(M, N, K, bits, group_size))
+        if (decode_shares_blocks(N) && (!workspace || workspace_bytes < bw_qmatmul_workspace_bytes(M, N, K, bits, group_size)))
             return BW_ERR_WORKSPACE;
         rc = qmatmul_decode(x, x_dtype, M, N, K, qweight, s, z, b, out, out_dtype, bits, group_size, workspace, st);
         if (rc != BW_ERR_UNSUPPORTED || paired) return rc;   // otherwise nothing was launched: use the cluster split-K kernel

@@ -905,6 +905,7 @@ int launch_dec(const DecMaps &maps, DecParams p, const Epilogue &ep, cudaStream_
     const size_t budget = (size_t)(g_dec.smem_kb > 0 ? g_dec.smem_kb : 224) * 1024;
     if (budget < fixed + 2 * stage) return BW_ERR_UNSUPPORTED;
     if (shared) {
+        if (!p.part || !aligned_to(p.part, 16)) return BW_ERR_WORKSPACE;
         p.cnt = counter_slice(p.part, dev, st);
         if (!p.cnt) {
             // no slice for this capture: the caller has another kernel, except for the gated epilogue, which
@@ -1017,12 +1018,17 @@ size_t decode_workspace_bytes(int64_t M, int64_t N, int64_t K, int bits) {
     return (size_t)2 * DK_MAX_CTAS * dec_token_tiles(M) * 8 * DK_ROWS * sizeof(float);
 }
 
+// Whether row blocks are shared through the scratch; a call that does not share them needs none.
+bool decode_shares_blocks(int64_t N) {
+    const int sms = sm_count();
+    return g_dec.max_ctas != 0 || (N + DK_ROWS - 1) / DK_ROWS > (sms < DK_MAX_CTAS ? sms : DK_MAX_CTAS);
+}
+
 // Returns BW_ERR_UNSUPPORTED (nothing launched) when no ring of two stages fits or no counters are free; the caller
 // then uses the cluster split-K kernel.
 int qmatmul_decode(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, const int32_t *q,
                    const __half *scale, const __half *zp, const __half *bias, void *out, int out_dtype,
                    int bits, int g, void *workspace, cudaStream_t st) {
-    if (!workspace || !aligned_to(workspace, 16)) return BW_ERR_WORKSPACE;
     const int vpi = 32 / bits, mt = dec_token_tiles(M);
     const int tile_k = DK_WORDS * vpi;
     DecParams p = {};

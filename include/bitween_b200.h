@@ -164,7 +164,8 @@ BW_API int bw_dequantize(const int32_t *qweight, const void *scale, int scale_dt
 BW_API size_t bw_qmatmul_workspace_bytes(int64_t M, int64_t N, int64_t K, int bits, int group_size);
 /* Same query for given activations: fp16 activations that start on a 16-byte boundary need no
  * cast for the tensor-core GEMM (x_align = the largest power of two, up to 16, dividing the
- * address of x), so large prefill calls need no workspace at all. */
+ * address of x), so large prefill calls need no workspace at all; up to 32 tokens the decode kernel's
+ * shares count only where the layer has more row blocks of 128 than the current device has SMs. */
 BW_API size_t bw_qmatmul_workspace_bytes_for(int64_t M, int64_t N, int64_t K, int bits, int group_size,
                                       int x_dtype, int x_align);
 

@@ -52,6 +52,9 @@ def test_status_strings_and_argument_validation_need_no_gpu():
     assert L.bw_qmatmul_workspace_bytes_for(4096, 4096, 4096, 4, 128, 1, 16) == 64 * 4096 * 2
     assert L.bw_qmatmul_workspace_bytes_for(4096, 4096, 4096, 4, 128, 2, 16) == 4096 * 4096 * 2
     assert L.bw_qmatmul_workspace_bytes_for(4096, 4096, 4096, 4, 128, 1, 2) == 4096 * 4096 * 2
+    # up to 32 tokens the decode kernel's shares count only with more row blocks than SMs (148 where no device is current)
+    assert L.bw_qmatmul_workspace_bytes_for(16, 4096, 4096, 4, 128, 1, 16) == 16 * 4096 * 2
+    assert L.bw_qmatmul_workspace_bytes_for(16, 128 * 149, 4096, 4, 128, 1, 16) == 2 * 160 * 16 * 128 * 4
     # fake quantization of the trainable mode: argument rules before any CUDA call
     assert L.bw_fake_quant(z, 0, 4, 64, 3, 32, z, z, z, 0, z, z, z) == 1
     assert L.bw_fake_quant(z, 0, 4, 48, 4, 32, z, z, z, 0, z, z, z) == 2

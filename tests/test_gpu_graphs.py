@@ -113,3 +113,22 @@ def test_counter_slices_are_given_back_with_their_graphs():
     torch.cuda.synchronize()
     assert kernel == anchor[1] == "qmm_decode_kernel" and torch.equal(out, want)
     assert _lib.lib().bw_device_status() == 0
+
+
+def test_scratch_of_the_decode_kernel_only_where_row_blocks_are_shared():
+    L = _lib.lib()
+    for N, K, rc in ((1024, 4096, 0), (148 * 128, 512, 0), (149 * 128, 512, _lib.ERR_WORKSPACE)):
+        q, s, z = _layer(N, K, 4, 64)
+        x = torch.randn(5, K, device=DEV).half()
+        out = torch.zeros(5, N, dtype=torch.float16, device=DEV)
+        want = quantized_matmul_cuda(x, q, s, z, None, 4, 64)
+        assert _lib.last_qmatmul_kernel() == "qmm_decode_kernel"
+        got = L.bw_qmatmul(x.data_ptr(), _lib.F16, 5, N, K, q.data_ptr(), s.data_ptr(), z.data_ptr(), None, out.data_ptr(), _lib.F16,
+                           4, 64, None, 0, _lib.raw_stream(x.device))
+        assert got == rc and torch.equal(out, want if rc == 0 else torch.zeros_like(want))
+    # a layout that runs on the cluster split-K kernel asks for its own scratch
+    q, s, z = _layer(64, 1408, 4, 128)
+    x = torch.randn(5, 1408, device=DEV).half()
+    assert L.bw_qmatmul_workspace_bytes_for(5, 64, 1408, 4, 128, _lib.F16, 16) >= 5 * 1408 * 2
+    quantized_matmul_cuda(x, q, s, z, None, 4, 128)
+    assert _lib.last_qmatmul_kernel() == "qmm_smallm_kernel"
