@@ -70,7 +70,8 @@ dequantize_kernel(const int32_t *__restrict__ qweight, const ST *__restrict__ sc
 // that vector stores can reach.  Rows are contiguous and hold whole groups, so the group of word wi is
 // wi >> log2(words per group): no divisions (two 64-bit ones a word above).  A thread takes four words
 // a block apart, all loads first: four independent chains in flight, loads and stores of a warp contiguous.
-// 4096 x 4096 W8 g32 -> fp32: 13.2 us (6.7 TB/s, the HBM rate) instead of 19.9.
+// 28672 x 8192 W8 g32 -> fp32: 198 us, 6.2 TB/s of inputs and outputs (0.95 of a plain copy's rate); 4096 x 4096, whose
+// outputs stay in L2, 15.9 us instead of 18.8.
 template <int BITS, typename ST, typename ZT, typename OutT>
 __global__ void __launch_bounds__(256)
 dequantize_words_kernel(const int32_t *__restrict__ qweight, const ST *__restrict__ scale, const ZT *__restrict__ zp,

@@ -11,8 +11,9 @@ What runs where on every training step (bitween/wrapper.py:116-172):
   * the per-group minima / maxima of the frozen weight are taken once at construction, not on
     every call (they cannot change: `orig_weight` is a buffer);
   * scale and float zero point come from them and the learnable factors on [N, K/group_size]
-    tensors with torch ops, so autograd tracks `min_scale` / `max_scale` exactly as in the
-    reference (clamp included);
+    tensors, clamp included: one kernel forward and one backward (`bw_group_params`), or the
+    same torch ops as in the reference where operands are not what the constructor made them
+    (no factors, another dtype, `_group_params` replaced) and under `create_graph`;
   * the [N,K] part -- divide, add, perturb, round, clamp, dequantize -- is `bw_fake_quant`, and
     its backward for (scale, zero_point) is `bw_fake_quant_backward`.
 The fused kernels compute in fp32, which is what the reference computes whenever an fp32

@@ -148,8 +148,9 @@ BW_API int bw_dequantize(const int32_t *qweight, const void *scale, int scale_dt
  *                   live graphs the cluster kernel runs).  Make the first call on a device
  *                   outside a stream capture (it looks up the address of the counters).
  * Accumulation is fp32.  The kernel is chosen from M and the layout: up to 32 tokens run on
- * the persistent TMA-fed decode kernel (one launch; needs K/group_size to be a multiple of 8
- * and 16-byte aligned rows, else the cluster split-K streaming kernel runs), more on the
+ * the persistent TMA-fed decode kernel (one launch; needs 16-byte aligned rows and K/group_size
+ * to be a multiple of 8, or, from 9 tokens on, a layer whose grid makes loading the scales
+ * directly pay; else the cluster split-K streaming kernel runs), more on the
  * tcgen05 tensor-core GEMM; unusual group sizes run on a slower general kernel, never on the
  * CPU.  The kernels are launched with programmatic dependent launch and fetch packed weights,
  * scales and zero points BEFORE waiting for the preceding kernel of the stream (only the
