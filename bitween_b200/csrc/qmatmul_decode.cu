@@ -36,6 +36,7 @@
 
 #include "bw_common.cuh"
 #include "qmm_dequant.cuh"
+#include "tensor_map.cuh"
 
 namespace bw {
 namespace {
@@ -707,33 +708,6 @@ qmm_decode_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
 }
 
 // ---- host side ---------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) == cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-    }
-    return fn;
-}
-
-int encode_2d(CUtensorMap *map, CUtensorMapDataType dt, const void *base, uint64_t inner, uint64_t outer,
-              uint64_t row_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swz) {
-    const cuuint64_t dims[2] = {inner, outer};
-    const cuuint64_t strides[1] = {row_bytes};
-    const cuuint32_t box[2] = {box_inner, box_outer};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode_tiled_fn()(map, dt, 2, const_cast<void *>(base), dims, strides, box, estr,
-                                         CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? BW_OK : BW_ERR_UNSUPPORTED;
-}
-
 struct DecTuning { int enabled, smem_kb, max_ctas, pdl; };
 DecTuning g_dec = {1, 0, 0, 1};
 
@@ -1050,17 +1024,15 @@ int qmatmul_decode(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, 
     // packed words [N rows][K/vpi int32]: boxes of 128 rows x 32 words, 128-byte swizzle; scales
     // and zero points [N rows][K/g fp16]: boxes of 128 rows x 8 groups; raw activations [M][K]:
     // boxes of 8*ceil(M/8) token slots x up to 256 k.  Everything outside a tensor arrives as zeros.
-    int rc = encode_2d(&maps.w, CU_TENSOR_MAP_DATA_TYPE_INT32, q, (uint64_t)(K / vpi), (uint64_t)N, (uint64_t)(K / vpi) * 4,
-                       DK_WORDS, DK_ROWS, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (!encode_2d(&maps.w, CU_TENSOR_MAP_DATA_TYPE_INT32, q, K / vpi, N, K / vpi * 4, DK_WORDS, DK_ROWS, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !encode_2d(&maps.x, x_dtype == BW_F32 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, x, K, M,
+                   K * (int64_t)dtype_size(x_dtype), tile_k < DK_XBOX ? tile_k : DK_XBOX, mt * 8, CU_TENSOR_MAP_SWIZZLE_NONE))
+        return BW_ERR_UNSUPPORTED;
     if (!ctma) maps.s = maps.z = maps.w;                  // not used
-    if (rc == BW_OK && ctma) rc = encode_2d(&maps.s, CU_TENSOR_MAP_DATA_TYPE_UINT16, scale, (uint64_t)(K / g), (uint64_t)N, (uint64_t)(K / g) * 2,
-                                    DK_GBOX, DK_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE);
-    if (rc == BW_OK && ctma) rc = encode_2d(&maps.z, CU_TENSOR_MAP_DATA_TYPE_UINT16, zp, (uint64_t)(K / g), (uint64_t)N, (uint64_t)(K / g) * 2,
-                                    DK_GBOX, DK_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE);
-    if (rc == BW_OK) rc = encode_2d(&maps.x, x_dtype == BW_F32 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, x,
-                                    (uint64_t)K, (uint64_t)M, (uint64_t)K * dtype_size(x_dtype),
-                                    (uint32_t)(tile_k < DK_XBOX ? tile_k : DK_XBOX), (uint32_t)(mt * 8), CU_TENSOR_MAP_SWIZZLE_NONE);
-    if (rc != BW_OK) return rc;
+    else if (!encode_2d(&maps.s, CU_TENSOR_MAP_DATA_TYPE_UINT16, scale, K / g, N, K / g * 2, DK_GBOX, DK_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+             !encode_2d(&maps.z, CU_TENSOR_MAP_DATA_TYPE_UINT16, zp, K / g, N, K / g * 2, DK_GBOX, DK_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE))
+        return BW_ERR_UNSUPPORTED;
+    int rc;
     switch (bits) {
         case 2: rc = launch_dec_ep<2>(maps, p, mt, ctma, st); break;
         case 4: rc = launch_dec_ep<4>(maps, p, mt, ctma, st); break;

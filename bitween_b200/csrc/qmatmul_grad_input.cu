@@ -20,6 +20,7 @@
 
 #include "bw_common.cuh"
 #include "qmm_dequant.cuh"
+#include "tensor_map.cuh"
 #include "umma.cuh"
 
 namespace cgx = cooperative_groups;
@@ -621,26 +622,6 @@ grad_input_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_c
     tc_fence_before();
     __syncthreads();
     if (warp == 3) tmem_dealloc(tmem_base, tmem_cols);
-}
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        const cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres);
-        return e == cudaSuccess && qres == cudaDriverEntryPointSuccess ? reinterpret_cast<EncodeTiledFn>(p) : nullptr;
-    }();
-    return fn;
-}
-bool encode_2d(CUtensorMap *map, CUtensorMapDataType dt, const void *base, int64_t inner, int64_t outer, int64_t row_bytes,
-               int box_inner, int box_outer, CUtensorMapSwizzle swz) {
-    const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer}, strides[1] = {(cuuint64_t)row_bytes};
-    const cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer}, estr[2] = {1, 1};
-    return encode_tiled_fn()(map, dt, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // Products that the mma.sync kernel does faster: one or two steps of weight rows and at most about two of its blocks an

@@ -40,6 +40,7 @@
 
 #include "bw_common.cuh"
 #include "qmm_dequant.cuh"
+#include "tensor_map.cuh"
 #include "umma.cuh"
 
 namespace cgx = cooperative_groups;
@@ -557,23 +558,7 @@ __global__ void __launch_bounds__(256) cast_to_f16_kernel(const XT *__restrict__
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 int g_tc_splits = 0;   // experiments: force the split-K factor (0 = automatic)
-
-EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) == cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-    }
-    return fn;
-}
 
 template <int BITS>
 int launch_tc(const CUtensorMap &xmap, const CUtensorMap &wmap, const CUtensorMap &omap, TcParams p, cudaStream_t st) {
@@ -730,26 +715,11 @@ int qmatmul_tc(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, cons
     p.pdl = direct ? 0 : 1;      // the cast kernel precedes this launch in the stream
     p.ep = current_epilogue();
 
-    CUtensorMap map;
-    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
-    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};                 // bytes between token rows
-    const cuuint32_t box[2] = {(cuuint32_t)TC_BK, (cuuint32_t)p.bn};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(xh), dims,
-                                         strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return BW_ERR_UNSUPPORTED;
-    // packed words: [N rows][K/vpi int32], one box = 128 rows x the words of one 64-k stage
-    CUtensorMap wmap;
-    const cuuint64_t wdims[2] = {(cuuint64_t)p.words_per_row, (cuuint64_t)N};
-    const cuuint64_t wstrides[1] = {(cuuint64_t)p.words_per_row * 4};
-    const cuuint32_t wbox[2] = {32u, (cuuint32_t)TC_BM};   // 128 bytes of every row: 2, 4 or 8 k-stages
-    const CUresult rw = encode_tiled_fn()(&wmap, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<int32_t *>(q), wdims,
-                                          wstrides, wbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rw != CUDA_SUCCESS) return BW_ERR_UNSUPPORTED;
+    CUtensorMap map, wmap;
+    // packed words: [N rows][K/vpi int32], one box = 128 rows x 128 bytes of every row (2, 4 or 8 k-stages)
+    if (!encode_2d(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, xh, K, M, K * 2, TC_BK, p.bn, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !encode_2d(&wmap, CU_TENSOR_MAP_DATA_TYPE_INT32, q, p.words_per_row, N, (int64_t)p.words_per_row * 4, 32, TC_BM, CU_TENSOR_MAP_SWIZZLE_128B))
+        return BW_ERR_UNSUPPORTED;
     // output [M tokens][N]: boxes of 32 tokens x 128 rows for the TMA-store epilogue (needs a 16-byte
     // aligned base and row pitch; a residual operand is read per element, so it takes the direct path)
     CUtensorMap omap = wmap;
@@ -758,14 +728,8 @@ int qmatmul_tc(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, cons
     // (token tiles of 64 and more: timed inside the kernel, the register-store epilogue of a 64-token tile
     // took 3 us of a 25 us launch)
     if (p.bn >= 64 && N >= TC_BM && (N * oes) % 16 == 0 && aligned_to(out, 16) && !p.ep.residual && p.ep.act != BW_ACT_SILU_MUL) {
-        const cuuint64_t odims[2] = {(cuuint64_t)N, (cuuint64_t)M};
-        const cuuint64_t ostrides[1] = {(cuuint64_t)N * oes};
-        const cuuint32_t obox[2] = {(cuuint32_t)TC_BM, 32u};
-        const CUresult ro = encode_tiled_fn()(&omap, out_dtype == BW_F32 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16,
-                                              2, out, odims, ostrides, obox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (ro == CUDA_SUCCESS) p.tma_store = 1;
+        p.tma_store = encode_2d(&omap, out_dtype == BW_F32 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, out, N, M,
+                                N * (int64_t)oes, TC_BM, 32, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE) ? 1 : 0;
     }
     set_last_kernel("qmm_tc_kernel");
     switch (bits) {
