@@ -939,30 +939,33 @@ static bool dec_const_tma(const void *scale, const void *zp, int64_t K, int g) {
     return (K / g) % 8 == 0 && aligned_to(scale, 16) && aligned_to(zp, 16);
 }
 // Others are loaded directly where that beats the cluster split-K kernel, from 9 tokens and 2^22 weights on.  Measured
-// over 770 random layers of 512..32768 rows and 1024..30000 columns (2 / 4 / 8 bits, groups of 32..128, 9..32 tokens,
+// over 1370 random layers of 512..32768 rows and 1024..30000 columns (2 / 4 / 8 bits, groups of 32..128, 9..32 tokens,
 // weights not in L2); below, us there / here:
 //   * the grid has to be resident at once; the chip holds 33 clusters of 4 and 15 of 8.  2048 x 8448, W4, 16 clusters of 8,
 //     14 tokens: 10.9 / 21.0;
-//   * idle SMs cost more here: 5248 x 25472, W8, 82 CTAs, 22 tokens: 106 / 132; 4096 x 9856, W4, 128 CTAs, 12 tokens:
-//     22.7 / 17.6.  Above 16 tokens the other kernel has two blocks a SM only, and at 2 and 4 bits this one wins from
-//     64 CTAs on: 5888 x 9024, W4, 92 CTAs, 29 tokens: 42.7 / 33.8;
-//   * a launch costs a fixed 6-8 us, which needs a few tiles a CTA: 11392 x 1280, W2, 3 tiles, 25 tokens: 10.1 / 13.0;
 //   * shares through the scratch (more row blocks than SMs) add 3-5 us: 30720 x 1536, W4, 22 tokens: 19.1 / 26.4;
-//     22912 x 5568: 70.2 / 54.8;
-//   * the other kernel cuts a row into 8 pieces at most: 768 x 21760, W4, 20 tokens: 34.4 / 21.8, whatever the grid.
-// In sum over all 1545 calls 0.84 of the other kernel's time (0.87 if all were taken, 0.82 for the better one each
-// time); 19 calls lose more than 8 %, none more than 19 %.
-static bool dec_direct_consts(int64_t M, int64_t N, int64_t K, int bits) {
+//     22912 x 5568: 70.2 / 54.8; with groups of 32 (more constants to stage there) 22784 x 4064, 27 tokens: 59.8 / 43.2;
+//   * from 48 row blocks on the other kernel has little to split: 10240 x 10496, W8, 21 tokens: 112 / 82; 12153 x 4160, W2,
+//     13 tokens: 27.3 / 19.2 (a tile or two a CTA do not cover the 6-8 us that a launch costs here);
+//   * with fewer, a grid that leaves SMs idle loses (4096 x 9856, W4, 128 CTAs, 12 tokens: 22.7 / 17.6; 3072 x 14592, 96 CTAs,
+//     10 tokens: 19.0 / 22.1), except above 16 tokens at 2 and 4 bits, where the other kernel has two blocks a SM only (5888
+//     x 9024, W4, 92 CTAs, 29 tokens: 42.7 / 33.8), with small groups (1536 x 8608, W4 g32, 30 tokens: 21.3 / 14.3) and in
+//     long rows, which it cuts into 8 pieces at most (768 x 21760, W4, 20 tokens: 34.4 / 21.8).
+// In sum over all 2718 calls 0.83 of the other kernel's time (0.87 if all were taken, 0.82 for the better one each
+// time); 102 lose more than 8 % (711 if all were taken).
+static bool dec_direct_consts(int64_t M, int64_t N, int64_t K, int bits, int g) {
     if (M <= 8 || N * K < (int64_t)1 << 22) return false;
     constexpr int64_t SMS = 148;
     const int64_t RB = (N + DK_ROWS - 1) / DK_ROWS, tile_k = DK_WORDS * (32 / bits), KT = (K + tile_k - 1) / tile_k;
-    if (RB > SMS) return K >= (M <= 16 ? 2560 : 5120);
+    if (RB > SMS) return K >= (M <= 16 ? 2560 : 5120) / (g <= 32 ? 2 : 1);
     const int per_rb = dec_ctas_per_block(RB, KT, SMS);
     if (RB > (per_rb == 8 ? 15 : (per_rb == 4 ? 33 : SMS))) return false;
     const int64_t ctas = RB * per_rb, tiles = (KT + per_rb - 1) / per_rb;
+    if (RB >= 48) return tiles >= 3;
     if (ctas >= 104 && tiles >= (bits == 8 ? 9 : 4)) return true;
-    if (M > 16 && bits < 8 && ctas >= 64 && tiles >= 5) return true;
-    return per_rb == 8 && K >= 16384;
+    if (M > 16 && bits < 8 && ctas >= 48 && tiles >= 4) return true;
+    if (g <= 32 && bits < 8 && ctas >= 80 && tiles >= 4) return true;
+    return (g * bits <= 256 && K >= 9216) || (per_rb == 8 && K >= 13056);
 }
 
 // Layout preconditions of the persistent decode kernel: at most 32 tokens, power-of-two groups
@@ -981,7 +984,7 @@ bool decode_path_ok(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K,
     if ((N + DK_ROWS - 1) / DK_ROWS * ((K / vpi + DK_WORDS - 1) / DK_WORDS) > (int64_t)1 << 30) return false;
     if (!aligned_to(q, 16)) return false;
     // (the gated epilogue is only offered where scales and zero points come by TMA)
-    if (!dec_const_tma(scale, zp, K, g) && (!dec_direct_consts(M, N, K, bits) || current_epilogue().act == BW_ACT_SILU_MUL)) return false;
+    if (!dec_const_tma(scale, zp, K, g) && (!dec_direct_consts(M, N, K, bits, g) || current_epilogue().act == BW_ACT_SILU_MUL)) return false;
     if (!aligned_to(x, 16) || (K * dtype_size(x_dtype)) % 16 != 0) return false;
     return encode_tiled_fn() != nullptr;
 }

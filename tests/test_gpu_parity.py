@@ -575,7 +575,8 @@ def test_persistent_decode_kernel_vs_oracle(case):
     # scratch (N > 148 * 128), ragged last k-tiles and row blocks
     (4, 128, 256, 16512, (9, 32)), (2, 64, 256, 16448, (9, 32)), (8, 128, 300, 16512, (9, 32)), (4, 128, 4000, 4480, (9, 32)),
     (8, 128, 3330, 4480, (9, 32)), (2, 128, 3330, 10368, (9, 32)), (4, 128, 6700, 2176, (9, 32)), (4, 128, 13400, 1152, (9, 32)),
-    (4, 128, 19200, 5248, (9, 32)), (8, 32, 20000, 2592, (9, 16)), (4, 128, 1000, 11008, (17, 32)),
+    (4, 128, 19200, 5248, (9, 32)), (8, 32, 20000, 2592, (9, 32)), (4, 128, 19200, 2688, (9, 16)), (4, 128, 1000, 11008, (17, 32)), (8, 128, 6200, 1664, (9, 32)),
+    (4, 64, 500, 9280, (9, 32)), (4, 32, 1300, 7200, (9, 32)), (4, 32, 19200, 2592, (9, 32)),
     # where the cluster split-K kernel is faster: few weights, few CTAs, few tiles, clusters that are not all resident
     (4, 32, 3300, 1312, None), (4, 64, 4000, 1088, None), (8, 128, 2978, 1408, None), (8, 128, 2979, 1408, None), (2, 64, 2048, 2112, None),
     (2, 128, 500, 8576, None), (4, 128, 19200, 1152, None), (8, 32, 20000, 544, None), (4, 128, 2048, 8448, None),
