@@ -65,6 +65,10 @@ int group_params(const void *w_min, const void *w_max, int dtype, const float *m
                  float *scale, float *zp, float *span, cudaStream_t st);
 int group_params_backward(const void *w_min, const void *w_max, int dtype, const float *scale, const float *zp, const float *span,
                           int64_t n, int bits, const float *gs, const float *gz, float *gmin, float *gmax, cudaStream_t st);
+bool rows_path_ok(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, const int32_t *q, int bits, int g);
+int qmatmul_rows(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, const int32_t *q,
+                 const __half *scale, const __half *zp, const __half *bias, void *out, int out_dtype,
+                 int bits, int g, cudaStream_t st);
 size_t peer_flag_bytes();
 size_t peer_state_bytes();
 int peer_device_status();
@@ -219,7 +223,20 @@ static int qmatmul_dispatch(const void *x, int x_dtype, int64_t M, int64_t N, in
     }
     if (!smallm_fast_path_ok(x, x_dtype, K, qweight, bits, group_size))
         return qmatmul_smallm(x, x_dtype, M, N, K, qweight, s, z, b, out, out_dtype, bits, group_size, nullptr, st);
-    if (persistent_decode && M <= 32 && decode_path_ok(x, x_dtype, M, N, K, qweight, scale, zero_point, bits, group_size)) {
+    const bool decode = persistent_decode && M <= 32 && decode_path_ok(x, x_dtype, M, N, K, qweight, scale, zero_point, bits, group_size);
+    // At most 8 tokens: the row kernel, but for layers of the decode kernel's layout that have more row blocks than SMs
+    // or, from 7 tokens on, 2^25 weights (8 tokens of bf16, 14336 x 4096, W4 g128: 13.6 us there, 14.4 here)
+    if (persistent_decode && rows_path_ok(x, x_dtype, M, N, K, qweight, bits, group_size) &&
+        !(decode && (decode_shares_blocks(N) || (M > 6 && N * K >= (int64_t)1 << 25)))) {
+        if (!decode && (!workspace || workspace_bytes < smallm_workspace_bytes(M, K, bits))) return BW_ERR_WORKSPACE;   // (as for the kernel that would take over)
+        rc = qmatmul_rows(x, x_dtype, M, N, K, qweight, s, z, b, out, out_dtype, bits, group_size, st);
+        if (rc == BW_OK) {
+            set_last_kernel(decode ? "qmm_decode_kernel" : "qmm_smallm_kernel");      // the family of layouts
+            note_launch("qmm_rows_kernel");
+        }
+        if (rc != BW_ERR_UNSUPPORTED) return rc;
+    }
+    if (decode) {
         if (decode_shares_blocks(N) && (!workspace || workspace_bytes < bw_qmatmul_workspace_bytes(M, N, K, bits, group_size)))
             return BW_ERR_WORKSPACE;
         rc = qmatmul_decode(x, x_dtype, M, N, K, qweight, s, z, b, out, out_dtype, bits, group_size, workspace, st);
