@@ -30,6 +30,10 @@ int rtn_quantize_pack_batch(const bw_rtn_job *jobs, int njobs, int w_dtype, int 
                             int zp_dtype, unsigned flags, void *table_dev, cudaStream_t st);
 int dequantize(const int32_t *q, const void *scale, int scale_dtype, const void *zp, int zp_dtype,
                int64_t N, int64_t K, int bits, int g, void *out, int out_dtype, cudaStream_t st);
+bool panel_path_ok(int64_t M, int bits, int g);
+int qmatmul_panel(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, const int32_t *q,
+                  const __half *scale, const __half *zp, const __half *bias, void *out, int out_dtype,
+                  int bits, int g, void *workspace, cudaStream_t st);
 int qmatmul_smallm(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, const int32_t *q,
                    const __half *scale, const __half *zp, const __half *bias, void *out, int out_dtype,
                    int bits, int g, void *workspace, cudaStream_t st);
@@ -235,6 +239,20 @@ static int qmatmul_dispatch(const void *x, int x_dtype, int64_t M, int64_t N, in
             note_launch("qmm_rows_kernel");
         }
         if (rc != BW_ERR_UNSUPPORTED) return rc;
+    }
+    // 9 to 32 tokens: the panel kernel, but for layers of the decode kernel's layout that have more row blocks than SMs or,
+    // above 16 tokens, more than 9472 rows (51 such layers of 4096..8192 columns: 1828 us there, 1982 here); without
+    // scratch for the prepared activations the decode kernel takes what it can
+    if (persistent_decode && panel_path_ok(M, bits, group_size) && !(decode && (decode_shares_blocks(N) || (M > 16 && N > 4 * 148 * 16)))) {
+        if (workspace && aligned_to(workspace, 16) && workspace_bytes >= smallm_workspace_bytes(M, K, bits)) {
+            rc = qmatmul_panel(x, x_dtype, M, N, K, qweight, s, z, b, out, out_dtype, bits, group_size, workspace, st);
+            if (rc == BW_OK) {
+                set_last_kernel(decode ? "qmm_decode_kernel" : "qmm_smallm_kernel");
+                note_launch("qmm_panel_kernel");
+            }
+            return rc;
+        }
+        if (!decode) return BW_ERR_WORKSPACE;
     }
     if (decode) {
         if (decode_shares_blocks(N) && (!workspace || workspace_bytes < bw_qmatmul_workspace_bytes(M, N, K, bits, group_size)))

@@ -35,6 +35,8 @@
 // weight prefetch of one layer overlaps the tail of the previous one.
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include "bw_common.cuh"
 #include "qmm_dequant.cuh"
 
@@ -495,6 +497,274 @@ int launch_xprep(const SmallMParams &p, int mt, uint4 *xp, cudaStream_t st) {
     }
 }
 
+
+// ---- panel kernel: 9 to 32 tokens -------------------------------------------------------------
+// The row kernel's form (qmatmul_rows.cu) for more tokens: a CTA owns 16, 32 or 64 whole rows, K is cut into one
+// contiguous range a warp, packed words go from memory to registers a block of chunks ahead, the warps' shares are
+// added at the end in the order of the k ranges, and the next launch's CTAs enter one by one with their words requested
+// before the wait.  The activations are not prepared by each CTA (16 tokens x 4096 would be 128 KB of its shared memory)
+// but once, by qmm_xprep_kernel, which runs beside the words' first loads; each lane reads its B fragments as they lie
+// there, 512 bytes a warp, from L1 and L2.
+// What bounds it: few rows a CTA read the activations often (tokens / 4 times the bytes of W4 words at 16 rows a
+// CTA), many rows leave SMs idle; with 4-byte sums for 32 tokens, registers.  Hence the rule on N in qmatmul_panel.
+// us in a graph, W4 g128, 16 tokens of bf16, ring kernel / this one: 4096 x 4096 8.8 / 6.0, 1024 x 4096 7.1 / 4.5,
+// 14336 x 4096 16.7 / 15.1, 4096 x 14336 16.7 / 15.7.  Sums over random layers of 2 / 4 / 8 bits and groups of 32..128,
+// the ring and cluster kernels / with this one: 1955 calls of 9..16 tokens 19.3 / 14.5 ms, 939 of 17..32 12.4 / 9.7 ms.
+struct PanelParams {
+    const uint4 *xp;      // prepared activations [chunks][NX][MT][32]
+    const uint4 *q;
+    const __half *scale, *zp, *bias;
+    void *out;
+    int64_t N, K;
+    int M;
+    int out_dtype;
+    int g_shift, G;
+    int vpr;              // 16-byte vectors per row of packed words
+    int chunks, cpw;      // k-chunks of a row, of a warp
+    int ne;               // groups of a block's table
+    int const_vec;        // groups can be read two at a time
+};
+// (predicated in place instead of branched around)
+__device__ __forceinline__ void pn_load(uint4 &v, const uint4 *p, bool live) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %5, 0;\n @p ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n}"
+                 : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w) : "l"(p), "r"((int)live));
+}
+// (not volatile, unlike mma_16816: the compiler may move the next word's dequantization between the MMAs)
+__device__ __forceinline__ void pn_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// RT row tiles of 16 a warp, WR warps along the rows, WK along k, blocks of D chunks.
+template <int BITS, int MT, int RT, int WR, int WK, int D, int OCC>
+__global__ void __launch_bounds__(WR * WK * 32, OCC)
+qmm_panel_kernel(const __grid_constant__ PanelParams p, const __grid_constant__ Epilogue ep) {
+    using Geo = Geometry<BITS>;
+    constexpr int R = RT * 16, ROWS = WR * R, RS = ROWS + 4, THREADS = WR * WK * 32, MTOK = MT * 8;
+    constexpr int LPR = 32 / R;                          // lanes that share a row's groups: 2 or 1
+    constexpr int NPF = 4;
+    extern __shared__ __align__(16) unsigned char pn_smem[];
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    const int wr = warp % WR, wk = warp / WR, g = lane >> 2, t = lane & 3;
+    const int64_t n0 = (int64_t)blockIdx.x * ROWS + wr * R;
+    const int c0 = min(wk * p.cpw, p.chunks), c1 = min(c0 + p.cpw, p.chunks);
+    const int lane_c1 = min(c1, (p.vpr - t + 3) / 4);
+    const uint4 *row[2 * RT];
+#pragma unroll
+    for (int s = 0; s < 2 * RT; ++s) row[s] = p.q + min(n0 + s * 8 + g, p.N - 1) * p.vpr + c0 * 4 + t;
+    uint4 w[D][2 * RT] = {};
+    int pc = c0;
+    auto request = [&](int d) {
+        const bool live = pc + d < lane_c1;
+#pragma unroll
+        for (int s = 0; s < 2 * RT; ++s) pn_load(w[d][s], row[s] + d * 4, live);
+    };
+    auto advance = [&]() {
+        pc += D;
+#pragma unroll
+        for (int s = 0; s < 2 * RT; ++s) row[s] += D * 4;
+    };
+#pragma unroll
+    for (int d = 0; d < D; ++d) request(d);
+    advance();
+    // constants of a block of D chunks, one block ahead
+    const int crow = lane % R, cpart = lane / R;
+    uint2 *const tab = reinterpret_cast<uint2 *>(pn_smem) + (size_t)warp * p.ne * R;
+    const unsigned short *srow, *zrow;
+    {
+        const int64_t n = min(n0 + crow, p.N - 1);
+        srow = reinterpret_cast<const unsigned short *>(p.scale) + n * p.G;
+        zrow = reinterpret_cast<const unsigned short *>(p.zp) + n * p.G;
+    }
+    auto first_group = [&](int c) { return (int)(((int64_t)c * Geo::KC) >> p.g_shift) & ~1; };
+    auto end_group = [&](int c) { return (int)((((int64_t)min(c + D, c1) * Geo::KC - 1) >> p.g_shift) + 1); };
+    uint32_t sv[NPF], zv[NPF];
+    auto pair_at = [&](const unsigned short *src, int e) {
+        if (p.const_vec) return e < p.G ? __ldg(reinterpret_cast<const uint32_t *>(src + e)) : 0u;
+        return (e < p.G ? (uint32_t)__ldg(src + e) : 0u) | (e + 1 < p.G ? (uint32_t)__ldg(src + e + 1) << 16 : 0u);
+    };
+    auto put = [&](int e, uint32_t s, uint32_t z) {
+        const __half2 k1024 = __float2half2_rn(1024.0f);
+        uint2 *d = tab + e * R + crow;
+        d[0] = make_uint2(__byte_perm(s, s, 0x1010), h2_as_u32(__hadd2(u32_as_h2(__byte_perm(z, z, 0x1010)), k1024)));
+        d[R] = make_uint2(__byte_perm(s, s, 0x3232), h2_as_u32(__hadd2(u32_as_h2(__byte_perm(z, z, 0x3232)), k1024)));
+    };
+    auto fetch_consts = [&](int c) {
+        if (c < c1) {
+            const int e0 = first_group(c), ng = end_group(c) - e0;
+#pragma unroll
+            for (int i = 0; i < NPF; ++i)
+                if (i * 2 * LPR < ng) { sv[i] = pair_at(srow, e0 + i * 2 * LPR + cpart * 2); zv[i] = pair_at(zrow, e0 + i * 2 * LPR + cpart * 2); }
+        }
+    };
+    auto store_consts = [&](int c) {
+        const int e0 = first_group(c), ng = end_group(c) - e0;
+#pragma unroll
+        for (int i = 0; i < NPF; ++i)
+            if (i * 2 * LPR < ng) put(i * 2 * LPR + cpart * 2, sv[i], zv[i]);
+        for (int e = NPF * 2 * LPR + cpart * 2; e < ng; e += 2 * LPR) put(e, pair_at(srow, e0 + e), pair_at(zrow, e0 + e));
+    };
+    fetch_consts(c0);
+
+    pdl_wait();
+    __threadfence();      // the scratch is reused from call to call: no line of it that this SM's L1 holds from before may answer
+    const uint4 *xl = p.xp + (size_t)c0 * Geo::NX * MT * 32 + lane;
+    float acc[RT][MT][4];
+#pragma unroll
+    for (int rt = 0; rt < RT; ++rt)
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[rt][mt][e] = 0.0f;
+
+    auto compute = [&](const uint4 (&v)[2 * RT], const uint2 *tb, int k) {
+        Dequant<BITS> dq[2 * RT];
+        auto set = [&](int kk) {
+            const uint2 *cs = tb + (kk >> p.g_shift) * R;
+#pragma unroll
+            for (int s = 0; s < 2 * RT; ++s) { const uint2 c = cs[s * 8]; dq[s].set(GroupConst{c.x, c.y}); }
+        };
+        set(k);
+        uint4 xq8[MT];
+        (void)xq8;
+#pragma unroll
+        for (int wi = 0; wi < 4; ++wi) {
+            if constexpr (BITS == 4) {
+                uint4 xf[MT];
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) xf[mt] = xl[(wi * MT + mt) * 32];
+#pragma unroll
+                for (int rt = 0; rt < RT; ++rt) {
+                    uint32_t qa[4], qb[4];
+                    dq[2 * rt].run((&v[2 * rt].x)[wi], qa);
+                    dq[2 * rt + 1].run((&v[2 * rt + 1].x)[wi], qb);
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt) pn_mma(acc[rt][mt], qa[0], qb[0], qa[1], qb[1], xf[mt].x, xf[mt].y);
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt) pn_mma(acc[rt][mt], qa[2], qb[2], qa[3], qb[3], xf[mt].z, xf[mt].w);
+                }
+            } else if constexpr (BITS == 8) {
+                if ((wi & 1) == 0) {
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt) xq8[mt] = xl[((wi >> 1) * MT + mt) * 32];
+                }
+#pragma unroll
+                for (int rt = 0; rt < RT; ++rt) {
+                    uint32_t qa[2], qb[2];
+                    dq[2 * rt].run((&v[2 * rt].x)[wi], qa);
+                    dq[2 * rt + 1].run((&v[2 * rt + 1].x)[wi], qb);
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt)
+                        pn_mma(acc[rt][mt], qa[0], qb[0], qa[1], qb[1], wi & 1 ? xq8[mt].z : xq8[mt].x, wi & 1 ? xq8[mt].w : xq8[mt].y);
+                }
+            } else {
+                if (wi == 2 && (1 << p.g_shift) < Geo::KL) set(k + Geo::KL / 2);
+                uint32_t qa[RT][8], qb[RT][8];
+#pragma unroll
+                for (int rt = 0; rt < RT; ++rt) {
+                    dq[2 * rt].run((&v[2 * rt].x)[wi], qa[rt]);
+                    dq[2 * rt + 1].run((&v[2 * rt + 1].x)[wi], qb[rt]);
+                }
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) {
+                    const uint4 xa = xl[(2 * wi * MT + mt) * 32], xb = xl[((2 * wi + 1) * MT + mt) * 32];
+#pragma unroll
+                    for (int rt = 0; rt < RT; ++rt) {
+                        pn_mma(acc[rt][mt], qa[rt][0], qb[rt][0], qa[rt][1], qb[rt][1], xa.x, xa.y);
+                        pn_mma(acc[rt][mt], qa[rt][2], qb[rt][2], qa[rt][3], qb[rt][3], xa.z, xa.w);
+                        pn_mma(acc[rt][mt], qa[rt][4], qb[rt][4], qa[rt][5], qb[rt][5], xb.x, xb.y);
+                        pn_mma(acc[rt][mt], qa[rt][6], qb[rt][6], qa[rt][7], qb[rt][7], xb.z, xb.w);
+                    }
+                }
+            }
+        }
+        xl += Geo::NX * MT * 32;
+    };
+    int k = c0 * Geo::KC + t * Geo::KL;
+    for (int c = c0; c < c1; c += D) {
+        __syncwarp();
+        store_consts(c);
+        __syncwarp();
+        fetch_consts(c + D);
+        const uint2 *tb = tab + g - first_group(c) * R;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            if (c + d < c1) { compute(w[d], tb, k); k += Geo::KC; }
+            request(d);
+        }
+        advance();
+    }
+    __syncthreads();      // (the tables are done with)
+    float *red = reinterpret_cast<float *>(pn_smem);     // [WK][MTOK][RS]
+#pragma unroll
+    for (int rt = 0; rt < RT; ++rt)
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                red[(wk * MTOK + mt * 8 + 2 * t + (e & 1)) * RS + wr * R + rt * 16 + (e >> 1) * 8 + g] = acc[rt][mt][e];
+    __syncthreads();
+    for (int i = threadIdx.x; i < p.M * ROWS; i += THREADS) {
+        const int m = i / ROWS, r = i % ROWS;
+        float v = 0.0f;
+#pragma unroll
+        for (int q = 0; q < WK; ++q) v += red[(q * MTOK + m) * RS + r];
+        const int64_t n = (int64_t)blockIdx.x * ROWS + r;
+        if (n < p.N) store_output(p.out, p.out_dtype, m * p.N + n, v, p.bias != nullptr, p.bias ? p.bias[n] : __half(), ep);
+    }
+}
+
+template <int BITS, int MT, int RT, int WR, int WK, int D, int OCC>
+int launch_panel(PanelParams p, cudaStream_t st) {
+    using Geo = Geometry<BITS>;
+    constexpr int R = RT * 16, ROWS = WR * R;
+    p.chunks = (int)((p.K + Geo::KC - 1) / Geo::KC);
+    p.cpw = (p.chunks + WK - 1) / WK;
+    if (p.cpw > 1) p.cpw = (p.cpw + 1) / 2 * 2;          // (blocks start on even groups at a chunk a group)
+    p.ne = ((D * Geo::KC - 1) >> p.g_shift) + 6;
+    const size_t tab = (size_t)WR * WK * p.ne * R * 8, red = (size_t)WK * MT * 8 * (ROWS + 4) * 4;
+    const size_t smem = tab > red ? tab : red;
+    auto kern = qmm_panel_kernel<BITS, MT, RT, WR, WK, D, OCC>;
+    constexpr size_t MOST = 227 * 1024 / OCC - 1024;
+    int dev = 0;
+    BW_CUDA_TRY(cudaGetDevice(&dev));
+    if (smem > MOST || dev < 0 || dev >= 64) return BW_ERR_UNSUPPORTED;
+    static std::atomic<bool> configured[64];             // per instantiation and device
+    if (!configured[dev].load(std::memory_order_relaxed)) {
+        BW_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST));
+        configured[dev].store(true, std::memory_order_relaxed);
+    }
+    return launch_ex(kern, dim3((unsigned)((p.N + ROWS - 1) / ROWS)), dim3(WR * WK * 32), smem, 1, st, p, current_epilogue());
+}
+
+// The shape of a CTA by the rows: row tiles of 16 fill the 148 SMs up to 2368 rows, 16 warps a tile then shorten the chain;
+// from there on fewer warps a tile, then more rows a CTA.  Sums in us over the random layers above, old kernels / 16 rows
+// and 16 warps / 16 rows and 8 warps / 32 rows / 64 rows:
+//   9..16 tokens: up to 2368 rows 6766 / 4558 / 5116 / 6707 / 9345, to 4736 4110 / 3933 / 2869 / 4127 / 6283,
+//   to 9472 4654 / 4632 / 4200 / 3806 / 5761, more 3335 / 4262 / 3238 / 3192 / 2951;
+//   17..32 tokens: up to 2368 4101 / 2659 / 2818 / 3456 / 5053, to 4736 2762 / 2428 / 2819 / 2167 / 3433,
+//   to 9472 3229 / 2930 / 3469 / 3281 / 2925 (K from 8192 on 943 / 759 / 994 / 1026 / 963).
+template <int BITS, int MT>
+int launch_panel_rows(const PanelParams &p, cudaStream_t st) {
+    constexpr int OCC = MT <= 2 ? 2 : 1;
+    constexpr int64_t FULL = 148 * 16;
+    if (p.N <= FULL) return launch_panel<BITS, MT, 1, 1, 16, 2, 1>(p, st);
+    if (MT <= 2) {
+        if (p.N <= 2 * FULL) return launch_panel<BITS, MT, 1, 1, 8, 4, OCC>(p, st);
+        if (p.N <= 4 * FULL) return launch_panel<BITS, MT, 2, 1, 8, 2, OCC>(p, st);
+        return launch_panel<BITS, MT, 2, 2, 4, 2, OCC>(p, st);
+    }
+    if (p.N <= 2 * FULL || p.N > 4 * FULL) return launch_panel<BITS, MT, 2, 1, 8, 2, OCC>(p, st);
+    if (p.K >= 8192) return launch_panel<BITS, MT, 1, 1, 16, 2, 1>(p, st);
+    return launch_panel<BITS, MT, 2, 2, 4, 2, OCC>(p, st);
+}
+template <int BITS>
+int launch_panel_mt(const PanelParams &p, cudaStream_t st) {
+    return p.M <= 16 ? launch_panel_rows<BITS, 2>(p, st) : launch_panel_rows<BITS, 4>(p, st);
+}
+
 template <int BITS, int MT, int RT, int WARPS, bool TWO_GROUPS>
 int launch_cfg(SmallMParams p, cudaStream_t st) {
     using Geo = Geometry<BITS>;
@@ -621,6 +891,43 @@ size_t smallm_workspace_bytes(int64_t M, int64_t K, int bits) {
     const int kc = 16 * (32 / bits);
     const int64_t mtok = M <= 8 ? 8 : (M <= 16 ? 16 : (M <= 32 ? 32 : 64));
     return (size_t)((K + kc - 1) / kc * kc) * mtok * 2;
+}
+
+// What the panel kernel takes of the layouts that smallm_fast_path_ok accepts: groups that hold a lane's vector of codes
+// (2 bits: half of one).
+bool panel_path_ok(int64_t M, int bits, int g) {
+    return M > 8 && M <= 32 && g >= (bits == 2 ? 32 : 128 / bits) && current_epilogue().act != BW_ACT_SILU_MUL;
+}
+
+// Prepares the activations in `workspace` (smallm_workspace_bytes) and runs the panel kernel; layouts of panel_path_ok.
+int qmatmul_panel(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, const int32_t *q,
+                  const __half *scale, const __half *zp, const __half *bias, void *out, int out_dtype,
+                  int bits, int g, void *workspace, cudaStream_t st) {
+    if (!workspace || !aligned_to(workspace, 16)) return BW_ERR_WORKSPACE;
+    SmallMParams prep = {};
+    prep.x = x; prep.M = M; prep.K = K; prep.x_dtype = x_dtype;
+    const int kc = 16 * (32 / bits), mt = M <= 16 ? 2 : 4;
+    prep.chunks_total = (int)((K + kc - 1) / kc);
+    uint4 *xp = reinterpret_cast<uint4 *>(workspace);
+    PanelParams p = {};
+    p.xp = xp; p.q = reinterpret_cast<const uint4 *>(q); p.scale = scale; p.zp = zp; p.bias = bias; p.out = out;
+    p.M = (int)M; p.N = N; p.K = K; p.out_dtype = out_dtype;
+    while ((1 << p.g_shift) < g) ++p.g_shift;
+    p.G = (int)(K / g);
+    p.vpr = (int)(K * bits / 128);
+    p.const_vec = p.G % 2 == 0 && aligned_to(scale, 4) && aligned_to(zp, 4);
+    int rc;
+    switch (bits) {
+        case 2: rc = launch_xprep<2>(prep, mt, xp, st); break;
+        case 4: rc = launch_xprep<4>(prep, mt, xp, st); break;
+        default: rc = launch_xprep<8>(prep, mt, xp, st); break;
+    }
+    if (rc != BW_OK) return rc;
+    switch (bits) {
+        case 2: return launch_panel_mt<2>(p, st);
+        case 4: return launch_panel_mt<4>(p, st);
+        default: return launch_panel_mt<8>(p, st);
+    }
 }
 
 // One launch pair (prepare + stream) for up to 64 tokens (the caller loops over token

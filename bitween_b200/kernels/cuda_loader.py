@@ -107,10 +107,14 @@ def quantized_matmul_cuda(x, qweight, scale, zero_point, bias, bits, group_size,
 
 def _launch(dev, args, ep, x_code):
     """bw_qmatmul on the current stream with the stream's workspace.  The size a call needs is only asked for
-    when the library reports that the workspace at hand is too small (nothing has been launched then)."""
+    when the library reports that the workspace at hand is too small (nothing has been launched then), or when
+    it would run without one on a slower kernel (9 to 32 tokens, whose activations are prepared in it)."""
     L = _lib.lib()
     stream = _lib.raw_stream(dev)
     ws = _lib.current_workspace(dev, stream)
+    M, _, K = args[2:5]
+    if 8 < M <= 32 and (ws is None or ws.numel() < 64 * (K + 256)):
+        ws = _lib.workspace(dev, L.bw_qmatmul_workspace_bytes_for(*args[2:5], args[11], args[12], x_code, 16 if args[0] % 16 == 0 else 2))
     while True:
         tail = (None, 0, stream) if ws is None else (ws.data_ptr(), ws.numel(), stream)
         rc = L.bw_qmatmul(*args, *tail) if ep is None else L.bw_qmatmul_fused(*args, ep, *tail)

@@ -1,4 +1,5 @@
-"""The kernel for at most 8 tokens: edges of its row tiles, k-chunks, warps' k ranges and constant tables, against float64."""
+"""The kernels for at most 8 and for 9 to 32 tokens: edges of their row tiles, k-chunks, warps' k ranges and constant
+tables, against float64."""
 import pytest
 import torch
 
@@ -52,18 +53,64 @@ def test_rows_kernel_matches_float64(bits, g, N, K, offset):
     assert ran >= 3
 
 
-def test_rows_kernel_of_calls_that_feed_each_other():
+@pytest.mark.parametrize("bits,g,N,K,offset", [
+    # 16 rows a CTA, 16 warps: less than a chunk, ragged chunks, odd groups, groups wider and narrower than a chunk
+    (4, 32, 1, 32, 0), (8, 16, 33, 80, 0), (2, 64, 31, 320, 0), (4, 128, 2368, 1408, 0), (2, 32, 50, 1088, 0), (8, 256, 70, 2304, 0), (4, 32, 200, 11008, 0),
+    # 16 rows and 8 warps or 32 rows; 32 or 64 rows, long rows; 64 or 32 rows: ragged last tiles
+    (4, 128, 2369, 1408, 0), (8, 32, 2400, 608, 0), (2, 32, 4736, 1152, 0), (4, 64, 4737, 576, 0), (8, 128, 4750, 1280, 0), (2, 128, 4800, 9344, 0),
+    (4, 128, 9472, 1408, 0), (4, 32, 9473, 672, 0), (8, 64, 9500, 448, 0), (2, 64, 19000, 448, 0), (4, 512, 9490, 1536, 0),
+    # scales and zero points off a 4-byte boundary
+    (4, 128, 300, 2048, 1), (8, 64, 4790, 1216, 3),
+])
+def test_panel_kernel_matches_float64(bits, g, N, K, offset):
+    gen = torch.Generator(device=DEV).manual_seed(N + K + bits)
+    q, s, z = _layer(N, K, bits, g, gen, offset)
+    b = torch.randn(N, generator=gen, device=DEV).half()
+    w = dequantize_rtn(q, s.contiguous(), z.contiguous(), g, bits=bits).half().double()
+    ran = 0
+    for M, xdt in ((9, torch.float16), (16, torch.bfloat16), (13, torch.float32), (17, torch.float16), (32, torch.float32), (25, torch.bfloat16)):
+        x = torch.randn(M, K, generator=gen, device=DEV).to(xdt)
+        y = quantized_matmul_cuda(x, q, s, z, b if M % 2 else None, bits, g, out_dtype=torch.float32)
+        ran += _lib.last_kernel() == "qmm_panel_kernel"
+        xh = x.half().double()
+        ref = xh @ w.T + (b.double() if M % 2 else 0.0)
+        slack = 2.0 ** -23 * (K / 16 + 16) * (xh.abs() @ w.abs().T) + 1e-6
+        assert bool(((y.double() - ref).abs() <= slack).all()), (M, xdt, float((y.double() - ref).abs().max()))
+        assert torch.equal(y, quantized_matmul_cuda(x, q, s, z, b if M % 2 else None, bits, g, out_dtype=torch.float32))
+    # (above 16 tokens the ring kernel keeps the wide layers of its layouts)
+    assert ran == 6 or (ran == 3 and N > 9472)
+
+
+def test_panel_kernel_without_scratch_leaves_the_call_to_the_ring_kernel():
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    L = _lib.lib()
+    for K, rc in ((1024, 0), (1408, _lib.ERR_WORKSPACE)):
+        q, s, z = _layer(256, K, 4, 128, gen)
+        x = torch.randn(12, K, generator=gen, device=DEV).half()
+        want = quantized_matmul_cuda(x, q, s, z, None, 4, 128)
+        assert _lib.last_kernel() == "qmm_panel_kernel"
+        out = torch.zeros_like(want)
+        got = L.bw_qmatmul(x.data_ptr(), _lib.F16, 12, 256, K, q.data_ptr(), s.data_ptr(), z.data_ptr(), None, out.data_ptr(), _lib.F16,
+                           4, 128, None, 0, _lib.raw_stream(x.device))
+        assert got == rc
+        if rc == 0:
+            assert _lib.last_kernel() == "qmm_decode_kernel"
+            assert float((out.float() - want.float()).abs().max()) <= 2.0 ** -10 * float(want.float().abs().max())
+
+
+@pytest.mark.parametrize("tokens,kernel", [(3, "qmm_rows_kernel"), (12, "qmm_panel_kernel"), (30, "qmm_panel_kernel")])
+def test_calls_that_feed_each_other(tokens, kernel):
     # each call reads what the one before has just written, in place and in a graph: weights are requested before the
     # wait for the preceding kernel, activations and the residual after it
     gen = torch.Generator(device=DEV).manual_seed(7)
     layers = [_layer(1024, 1024, 4, 128, gen) for _ in range(6)]
     layers = [(q, s * 0.2, z) for q, s, z in layers]
-    h0 = torch.randn(3, 1024, generator=gen, device=DEV).half()
+    h0 = torch.randn(tokens, 1024, generator=gen, device=DEV).half()
 
     def run(h):
         for q, s, z in layers:
             quantized_matmul_cuda(h, q, s, z, None, 4, 128, residual=h.clone(), out=h)
-            assert _lib.last_kernel() == "qmm_rows_kernel"
+            assert _lib.last_kernel() == kernel
         return h
 
     want = h0.clone()
