@@ -1,5 +1,7 @@
 """Builds libbitween_b200.so in-tree with nvcc for sm_100a (no JIT cache, no torch headers).
 
+Beside it lands _host_forward, the native host side of the layer's forward (g++, torch's headers and libraries).
+
 Run as `python -m bitween_b200.csrc.build` or call build(); the library lands in
 bitween_b200/_C/ next to the Python package so that it travels with the source tree.
 """
@@ -15,6 +17,7 @@ ROOT = os.path.dirname(PKG)
 OUT_DIR = os.path.join(PKG, "_C")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(OUT_DIR, "libbitween_b200.so")
+HOST_LIB = os.path.join(OUT_DIR, "_host_forward.so")
 
 SOURCES = ["api.cu", "rtn_quantize.cu", "dequantize.cu", "qmatmul_smallm.cu", "qmatmul_rows.cu", "qmatmul_decode.cu", "qmatmul_tc.cu", "qmatmul_grad_input.cu", "fake_quant.cu", "peer_allreduce.cu"]
 
@@ -42,6 +45,27 @@ def _stale(target, deps):
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _build_host(force=False, verbose=False):
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    src = os.path.join(HERE, "host_forward.cpp")
+    if not force and not _stale(HOST_LIB, [src, os.path.join(ROOT, "include", "bitween_b200.h"), torch.__file__]):
+        return
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    includes = [os.path.join(ROOT, "include"), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]] + cpp_extension.include_paths()
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + \
+        [f"-I{d}" for d in includes] + [src, "-o", HOST_LIB, f"-L{libs}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+                                               "-L" + os.path.join(cuda, "lib64"), "-lcudart"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode != 0:
+        sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed for host_forward.cpp")
+
+
 def build(force=False, verbose=False, ptxas_info=False):
     os.makedirs(OUT_DIR, exist_ok=True)
     os.makedirs(OBJ_DIR, exist_ok=True)
@@ -62,6 +86,7 @@ def build(force=False, verbose=False, ptxas_info=False):
         r = subprocess.run(cmd, capture_output=True, text=True)
         return cmd, r
 
+    host = concurrent.futures.ThreadPoolExecutor(max_workers=1).submit(_build_host, force, verbose)
     if jobs:
         with concurrent.futures.ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 4)) as ex:
             for cmd, r in ex.map(run, jobs):
@@ -76,6 +101,7 @@ def build(force=False, verbose=False, ptxas_info=False):
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    host.result()
     return LIB
 
 

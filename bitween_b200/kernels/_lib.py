@@ -6,6 +6,7 @@ is absent) or no CUDA device is present, the calls raise.
 """
 import contextlib
 import ctypes
+import importlib.util
 import os
 import threading
 
@@ -140,6 +141,28 @@ def lib():
                 _declare(L)
                 _lib = L
     return _lib
+
+
+_host = None
+HOST_LIB_PATH = os.path.join(_PKG, "_C", "_host_forward.so")
+
+
+def host_forward():
+    """The native host side of a layer's forward (csrc/host_forward.cpp), loaded with the library and built with it."""
+    global _host
+    if _host is None:
+        L = lib()
+        with _lock:
+            if _host is None:
+                if not os.path.exists(HOST_LIB_PATH):
+                    from ..csrc.build import build
+                    build()
+                spec = importlib.util.spec_from_file_location("_host_forward", HOST_LIB_PATH)
+                module = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(module)
+                module.set_entry(ctypes.cast(L.bw_qmatmul, ctypes.c_void_p).value, _workspaces)
+                _host = module.forward
+    return _host
 
 
 def check(status):

@@ -6,6 +6,7 @@ import torch
 import torch.nn as nn
 
 from .functional import quantize_rtn_to_module_buffers
+from .kernels import _lib
 from .kernels.cuda_loader import quantized_matmul_cuda, quantized_matmul_grad_input
 
 
@@ -80,6 +81,11 @@ class QuantizedLinear(nn.Module):
                 or cls.__getattribute__ is not nn.Module.__getattribute__:
             out_dtype = getattr(self, "out_dtype", None)
         if out_dtype is None:
+            # plain calls that record no gradient, in one native call; None: everything else
+            if x.is_cuda:
+                y = (_lib._host or _lib.host_forward())(x, self.qweight, self.scale, self.zero_point, self.bias, self.bits, self.group_size)
+                if y is not None:
+                    return y
             return QuantizedLinearFunction.apply(x, self.qweight, self.scale, self.zero_point, self.bias,
                                                  self.bits, self.group_size)
         return QuantizedLinearFunction.apply(x, self.qweight, self.scale, self.zero_point, self.bias,
