@@ -205,8 +205,8 @@ static int qmatmul_validate(const void *x, int x_dtype, int64_t M, int64_t N, in
     return BW_OK;
 }
 
-// `persistent_decode`: let M <= 32 run on the persistent TMA-fed decode kernel (needs the larger
-// workspace of bw_qmatmul_workspace_bytes); otherwise only the cluster split-K streaming kernel
+// `persistent_decode`: let M <= 32 run on the row, panel and persistent TMA-fed decode kernels (the last needs the
+// larger workspace of bw_qmatmul_workspace_bytes); otherwise only the cluster split-K streaming kernel
 // and the tensor-core GEMM are used.  `allow_tc`: the tensor-core GEMM may be used (its
 // activation cast, where one is needed, fits the workspace).
 static int qmatmul_dispatch(const void *x, int x_dtype, int64_t M, int64_t N, int64_t K, const int32_t *qweight,
@@ -228,11 +228,18 @@ static int qmatmul_dispatch(const void *x, int x_dtype, int64_t M, int64_t N, in
     if (!smallm_fast_path_ok(x, x_dtype, K, qweight, bits, group_size))
         return qmatmul_smallm(x, x_dtype, M, N, K, qweight, s, z, b, out, out_dtype, bits, group_size, nullptr, st);
     const bool decode = persistent_decode && M <= 32 && decode_path_ok(x, x_dtype, M, N, K, qweight, scale, zero_point, bits, group_size);
-    // At most 8 tokens: the row kernel, but for layers of the decode kernel's layout that have more row blocks than SMs
-    // or, from 7 tokens on, 2^25 weights (8 tokens of bf16, 14336 x 4096, W4 g128: 13.6 us there, 14.4 here)
-    if (persistent_decode && rows_path_ok(x, x_dtype, M, N, K, qweight, bits, group_size) &&
-        !(decode && (decode_shares_blocks(N) || (M > 6 && N * K >= (int64_t)1 << 25)))) {
-        if (!decode && (!workspace || workspace_bytes < smallm_workspace_bytes(M, K, bits))) return BW_ERR_WORKSPACE;   // (as for the kernel that would take over)
+    // At most 8 tokens: the row kernel, but for some layers of the decode kernel's layout (us there / here, W4 g128):
+    //   * from 7 tokens on, 2^25 weights or more: 8 tokens of bf16, 14336 x 4096, 13.6 / 14.4;
+    //   * more row blocks than SMs (their shares travel through scratch there) with 2 bits (28672 x 1024, 1 token 9.4 / 10.4),
+    //     5 tokens or more (6 tokens, 28672 x 4096, 23.2 / 23.8; 24576 x 6144, W8, 34.9 / 53.6) or less than 2^24 weights;
+    //     otherwise 1 token 19200 x 2048 12.0 / 8.6, 28672 x 4096 22.7 / 18.5, 32768 x 8192 41.7 / 36.4, 3 tokens 41.8 / 37.1.
+    const bool wide = decode && decode_shares_blocks(N), many = N * K >= (int64_t)1 << 25;
+    const bool ring = (M > 6 && many) || (wide && (bits == 2 || M > 4 || N * K < (int64_t)1 << 24));
+    if (persistent_decode && rows_path_ok(x, x_dtype, M, N, K, qweight, bits, group_size) && !(decode && ring)) {
+        // (scratch is asked for wherever the kernel that would take over needs it)
+        if ((!decode || wide) && (!workspace || !aligned_to(workspace, 16))) return BW_ERR_WORKSPACE;
+        if (!decode && workspace_bytes < smallm_workspace_bytes(M, K, bits)) return BW_ERR_WORKSPACE;
+        if (wide && workspace_bytes < bw_qmatmul_workspace_bytes(M, N, K, bits, group_size)) return BW_ERR_WORKSPACE;
         rc = qmatmul_rows(x, x_dtype, M, N, K, qweight, s, z, b, out, out_dtype, bits, group_size, st);
         if (rc == BW_OK) {
             set_last_kernel(decode ? "qmm_decode_kernel" : "qmm_smallm_kernel");      // the family of layouts
@@ -240,10 +247,12 @@ static int qmatmul_dispatch(const void *x, int x_dtype, int64_t M, int64_t N, in
         }
         if (rc != BW_ERR_UNSUPPORTED) return rc;
     }
-    // 9 to 32 tokens: the panel kernel, but for layers of the decode kernel's layout that have more row blocks than SMs or,
-    // above 16 tokens, more than 9472 rows (51 such layers of 4096..8192 columns: 1828 us there, 1982 here); without
-    // scratch for the prepared activations the decode kernel takes what it can
-    if (persistent_decode && panel_path_ok(M, bits, group_size) && !(decode && (decode_shares_blocks(N) || (M > 16 && N > 4 * 148 * 16)))) {
+    // 9 to 32 tokens: the panel kernel, but for layers of the decode kernel's layout that have more row blocks than SMs (16
+    // tokens, 24576 x 6144, W4: 34.0 us there, 39.1 here), 2^26 weights of 2 bits (19 layers of 9..16 tokens: 587 / 612), or,
+    // above 16 tokens, more than 9472 rows (51 such layers of 4096..8192 columns: 1828 / 1982); without scratch for the
+    // prepared activations the decode kernel takes what it can
+    if (persistent_decode && panel_path_ok(M, bits, group_size) &&
+        !(decode && (wide || (bits == 2 && N * K >= (int64_t)1 << 26) || (M > 16 && N > 4 * 148 * 16)))) {
         if (workspace && aligned_to(workspace, 16) && workspace_bytes >= smallm_workspace_bytes(M, K, bits)) {
             rc = qmatmul_panel(x, x_dtype, M, N, K, qweight, s, z, b, out, out_dtype, bits, group_size, workspace, st);
             if (rc == BW_OK) {

@@ -1,3 +1,5 @@
+// The ring kernel of decode (most calls of up to 8 and of 9 to 32 tokens run on qmatmul_rows.cu and the panel kernel of
+// qmatmul_smallm.cu; this one takes the gated output stage and the layers that the dispatch in api.cu names).
 // Decode ("few tokens") quantized matmul for sm_100a: out[M,N] = x[M,K] . W[N,K]^T (+bias) for
 // M <= 32, W = fp16(scale * (code - zero_point)) bit-identical to the reference's dequantized
 // weights (bitween/modules.py:55-58), fp32 accumulation, fp16 output rounding and a separate
