@@ -52,13 +52,13 @@ LLAMA70B_LINEARS = [("q_proj", HIDDEN70, HIDDEN70, "column"), ("k_proj", KV70, H
                     ("gate_proj", FFN70, HIDDEN70, "column"), ("up_proj", FFN70, HIDDEN70, "column"),
                     ("down_proj", HIDDEN70, FFN70, "row")]
 
-# DRAM bytes of one qmm_decode_kernel launch (dram__bytes_read.sum + dram__bytes_write.sum of an ncu
-# capture of `bench.py --case decode:<shape>:<tokens>`, second captured launch) divided by its
-# algorithmic bytes, at 1 and 16 tokens per shape; token counts in between are interpolated.
+# DRAM bytes of one launch of the call's kernel (qmm_rows_kernel at 1 token, qmm_panel_kernel at 16;
+# dram__bytes_read.sum + dram__bytes_write.sum of an ncu capture of `bench.py --case
+# decode:<shape>:<tokens>`, second captured launch) divided by its algorithmic bytes, at 1 and 16 tokens per shape; token counts in between are interpolated.
 # Constants from those captures, not measured during the run.  Below 1.0: the outputs (and part of
 # the activations) never leave L2 within the launch.
-DECODE_TRAFFIC_FACTOR = {"q_o_proj": {1: 1.0064, 16: 0.9937}, "kv_proj": {1: 1.0285, 16: 1.0170},
-                         "gate_up_proj": {1: 1.0012, 16: 0.9881}, "down_proj": {1: 1.0019, 16: 0.9982}}
+DECODE_TRAFFIC_FACTOR = {"q_o_proj": {1: 1.0039, 16: 0.9889}, "kv_proj": {1: 1.0184, 16: 0.9954},
+                         "gate_up_proj": {1: 1.0005, 16: 0.9864}, "down_proj": {1: 1.0011, 16: 0.9968}}
 
 
 def decode_traffic_factor(name, M):
@@ -275,7 +275,8 @@ def run_decode8b(args, torch, dist, rank, world, device):
                     quantized_matmul_cuda(xs[M][L.K], L.q, L.scale, L.zp, None, bits, g, out=outs[M][L.N])
 
     calls_per_step = len(DECODE_M) * args.layers * len(LLAMA8B_SHAPES)
-    launches_per_step = calls_per_step                      # the decode kernel is the only launch of a call
+    # one launch a call, and from 9 tokens on one more that prepares the activations
+    launches_per_step = sum(2 if M > 8 else 1 for M in DECODE_M) * args.layers * len(LLAMA8B_SHAPES)
     per_shape = {name: sum(decode_bytes(M, N, K, bits, g) for M in DECODE_M) for (name, N, K) in LLAMA8B_SHAPES}
     bytes_per_step = sum(per_shape.values()) * args.layers
     traffic_per_step = sum(decode_bytes(M, N, K, bits, g) * decode_traffic_factor(name, M)
@@ -530,7 +531,7 @@ def run_case(args, torch, device):
     for L in layers:                       # warm-up pass (also the launches a profiler skips)
         body(L)
     ms = time_region(torch, lambda: [body(L) for L in layers]) / copies
-    print(json.dumps({"case": args.case, "kernel": _lib.last_qmatmul_kernel() if kind in ("decode", "prefill") else kind,
+    print(json.dumps({"case": args.case, "kernel": _lib.last_kernel() if kind in ("decode", "prefill") else kind,
                       "us_per_launch": round(ms * 1e3, 2), "copies": copies,
                       "note": "plain launches, back to back, no L2 flush: a profiling aid, not a benchmark value"}), flush=True)
 
@@ -816,7 +817,7 @@ def main():
 
     if rank == 0:
         peaks = read_peaks()
-        # the roofline is stated per qmatmul call (one launch of the decode kernel), its duration
+        # the roofline is stated per qmatmul call, its duration
         # the call's share of the timed region
         ms_per_launch = res["ms"] / max(res["calls"], 1)
         achieved = res["bytes_per_launch"] / (ms_per_launch * 1e-3) / 1e9
