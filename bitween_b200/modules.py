@@ -82,7 +82,7 @@ class QuantizedLinear(nn.Module):
             out_dtype = getattr(self, "out_dtype", None)
         if out_dtype is None:
             # plain calls that record no gradient, in one native call; None: everything else
-            if x.is_cuda:
+            if type(x) is torch.Tensor and x.is_cuda:
                 y = (_lib._host or _lib.host_forward())(x, self.qweight, self.scale, self.zero_point, self.bias, self.bits, self.group_size)
                 if y is not None:
                     return y
