@@ -744,6 +744,9 @@ int launch_panel(PanelParams p, cudaStream_t st) {
 // and 16 warps / 16 rows and 8 warps / 32 rows / 64 rows:
 //   9..16 tokens: up to 2368 rows 6766 / 4558 / 5116 / 6707 / 9345, to 4736 4110 / 3933 / 2869 / 4127 / 6283,
 //   to 9472 4654 / 4632 / 4200 / 3806 / 5761, more 3335 / 4262 / 3238 / 3192 / 2951;
+//   of those, 96 rows a CTA and 12 warps up to 14208 rows, one CTA an SM: 64 rows / 96 rows, 16 tokens, 11008 x 4096: W4 g128
+//   14.6 / 13.5, W4 g32 22.0 / 17.7, W8 g128 18.8 / 18.0, W2 g64 18.2 / 13.3 (registers; 128 of them spill at 2 bits, one CTA
+//   of 64 rows an SM is slower still); 14208 x 1024, W4 g32 6.0 / 6.5;
 //   17..32 tokens: up to 2368 4101 / 2659 / 2818 / 3456 / 5053, to 4736 2762 / 2428 / 2819 / 2167 / 3433,
 //   to 9472 3229 / 2930 / 3469 / 3281 / 2925 (K from 8192 on 943 / 759 / 994 / 1026 / 963).
 template <int BITS, int MT>
@@ -751,9 +754,10 @@ int launch_panel_rows(const PanelParams &p, cudaStream_t st) {
     constexpr int OCC = MT <= 2 ? 2 : 1;
     constexpr int64_t FULL = 148 * 16;
     if (p.N <= FULL) return launch_panel<BITS, MT, 1, 1, 16, 2, 1>(p, st);
-    if (MT <= 2) {
+    if constexpr (MT <= 2) {
         if (p.N <= 2 * FULL) return launch_panel<BITS, MT, 1, 1, 8, 4, OCC>(p, st);
         if (p.N <= 4 * FULL) return launch_panel<BITS, MT, 2, 1, 8, 2, OCC>(p, st);
+        if (p.N <= 6 * FULL && (BITS == 2 || p.K >= 1536)) return launch_panel<BITS, MT, 2, 3, 4, 2, 1>(p, st);
         return launch_panel<BITS, MT, 2, 2, 4, 2, OCC>(p, st);
     }
     if (p.N <= 2 * FULL || p.N > 4 * FULL) return launch_panel<BITS, MT, 2, 1, 8, 2, OCC>(p, st);

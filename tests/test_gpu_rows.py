@@ -60,7 +60,9 @@ def test_rows_kernel_matches_float64(bits, g, N, K, offset):
     (4, 32, 1, 32, 0), (8, 16, 33, 80, 0), (2, 64, 31, 320, 0), (4, 128, 2368, 1408, 0), (2, 32, 50, 1088, 0), (8, 256, 70, 2304, 0), (4, 32, 200, 11008, 0),
     # 16 rows and 8 warps or 32 rows; 32 or 64 rows, long rows; 64 or 32 rows: ragged last tiles
     (4, 128, 2369, 1408, 0), (8, 32, 2400, 608, 0), (2, 32, 4736, 1152, 0), (4, 64, 4737, 576, 0), (8, 128, 4750, 1280, 0), (2, 128, 4800, 9344, 0),
-    (4, 128, 9472, 1408, 0), (4, 32, 9473, 672, 0), (8, 64, 9500, 448, 0), (2, 64, 19000, 448, 0), (4, 512, 9490, 1536, 0),
+    (4, 128, 9472, 1408, 0), (4, 32, 9473, 672, 0), (8, 64, 9500, 448, 0), (2, 64, 19000, 448, 0),
+    # 96 rows a CTA
+    (4, 512, 9490, 1536, 0), (8, 64, 9505, 1600, 0), (2, 32, 14208, 448, 0),
     # scales and zero points off a 4-byte boundary
     (4, 128, 300, 2048, 1), (8, 64, 4790, 1216, 3),
 ])
