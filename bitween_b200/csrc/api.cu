@@ -2,6 +2,7 @@
 // argument validation, status codes and kernel dispatch.  No torch types, no allocation.
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 #include "bw_common.cuh"
 
@@ -87,6 +88,15 @@ int qmatmul_grad_input(const void *go, int dtype, int64_t M, int64_t N, int64_t 
 // Token counts above this go to the tensor-core GEMM, the rest to the streaming kernels.
 static int64_t g_tc_min_tokens = 32;
 #define TC_MIN_TOKENS g_tc_min_tokens
+
+// The lock under which a call enqueues the kernels that use its scratch.  Stream order alone keeps single launches
+// apart, not the pairs that hand prepared or cast activations over in scratch: a second thread on the same stream with
+// the same scratch could put a launch of its own between the two.  Chosen by address, so that calls with scratch of
+// their own seldom meet; it is held for the launches alone (a few us), never while anything is waited for.
+static std::mutex &scratch_lock(const void *workspace) {
+    static std::mutex locks[64];
+    return locks[(reinterpret_cast<uintptr_t>(workspace) >> 9) % 64];
+}
 
 static bool is_float_dtype(int dt) { return dt == BW_F32 || dt == BW_F16 || dt == BW_BF16; }
 
@@ -247,6 +257,8 @@ static int qmatmul_dispatch(const void *x, int x_dtype, int64_t M, int64_t N, in
         }
         if (rc != BW_ERR_UNSUPPORTED) return rc;
     }
+    std::unique_lock<std::mutex> together;
+    if (workspace) together = std::unique_lock<std::mutex>(scratch_lock(workspace));
     // 9 to 32 tokens: the panel kernel, but for layers of the decode kernel's layout that have more row blocks than SMs (16
     // tokens, 24576 x 6144, W4: 34.0 us there, 39.1 here), 2^26 weights of 2 bits (19 layers of 9..16 tokens: 587 / 612), or,
     // above 16 tokens, more than 9472 rows (51 such layers of 4096..8192 columns: 1828 / 1982); without scratch for the

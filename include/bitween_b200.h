@@ -140,6 +140,7 @@ BW_API int bw_dequantize(const int32_t *qweight, const void *scale, int scale_dt
  *                   BW_F32: acc + bias with no 16-bit rounding (fp32-accumulate checks)
  *   workspace       device scratch of at least bw_qmatmul_workspace_bytes(...) bytes, or
  *                   NULL when that is 0.  Calls that overlap on the GPU must not share it;
+ *                   threads that call on one stream may (a call's launches stay together there);
  *                   a call captured into a CUDA graph runs whenever the graph is replayed,
  *                   so graphs that may be replayed beside each other need a workspace each.
  *                   The decode kernel's row-block counters are the library's: outside
