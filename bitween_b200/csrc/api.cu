@@ -368,15 +368,14 @@ size_t bw_qmatmul_noalloc_max_scratch_bytes(void) {
 // small kernel instead -- plain 16-byte loads / stores on the host buffer's device mapping
 // (pinned memory is mapped into the unified address space), launched with programmatic
 // stream serialisation so that its launch latency overlaps its predecessor.
-__global__ void __launch_bounds__(256) staging_copy_kernel(const unsigned char *__restrict__ src,
-                                                           unsigned char *__restrict__ dst, size_t bytes) {
+__global__ void __launch_bounds__(256) staging_copy_kernel(const unsigned char *src, unsigned char *dst, size_t bytes) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");      // dst may still be read, src still be written, by the predecessor
     const size_t n16 = bytes / 16;
     const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = tid; i < n16; i += stride)
-        reinterpret_cast<uint4 *>(dst)[i] = reinterpret_cast<const uint4 *>(src)[i];
-    for (size_t i = n16 * 16 + tid; i < bytes; i += stride) dst[i] = src[i];
+        reinterpret_cast<uint4 *>(dst)[i] = __ldcg(reinterpret_cast<const uint4 *>(src) + i);   // (from L2: see bw_common.cuh)
+    for (size_t i = n16 * 16 + tid; i < bytes; i += stride) dst[i] = __ldcg(src + i);
 }
 
 // The device-side address of a pinned (mapped) host buffer, or nullptr.

@@ -68,6 +68,10 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(flo
 // kernel, bitween/modules.py:100-101): activation (ReLU, the OPT feed-forward) and residual add.
 // fp16 outputs reproduce the eager op-by-op result: fp16(acc), + bias, relu, + residual, each
 // rounded to fp16 like the separate torch ops would.
+//
+// What the kernels before may have written (activations, a residual) is read from L2, never through L1 or as read-only
+// data: a grid launched programmatically is resident while its predecessors still write, and its SM's L1, emptied when it
+// entered, may hold lines that a grid before the last has read since.
 struct Epilogue {
     int act;                  // BW_ACT_NONE | BW_ACT_RELU | BW_ACT_SILU_MUL
     const __half *residual;   // [M, N] fp16, added last, or null
@@ -81,12 +85,12 @@ __device__ __forceinline__ void store_output(void *out, int out_dtype, int64_t i
         __half c = __float2half_rn(v);                       // the GEMM's fp16 output rounding
         if (has_bias) c = __hadd(c, bias);                   // separate fp16 bias add
         if (ep.act == BW_ACT_RELU) c = __hmax(c, __float2half(0.0f));
-        if (ep.residual) c = __hadd(c, ep.residual[idx]);
+        if (ep.residual) c = __hadd(c, __ldcg(ep.residual + idx));
         reinterpret_cast<__half *>(out)[idx] = c;
     } else {
         if (has_bias) v += __half2float(bias);
         if (ep.act == BW_ACT_RELU) v = fmaxf(v, 0.0f);
-        if (ep.residual) v += __half2float(ep.residual[idx]);
+        if (ep.residual) v += __half2float(__ldcg(ep.residual + idx));
         if (out_dtype == BW_BF16) reinterpret_cast<__nv_bfloat16 *>(out)[idx] = __float2bfloat16_rn(v);
         else reinterpret_cast<float *>(out)[idx] = v;
     }
@@ -104,12 +108,12 @@ __device__ __forceinline__ void store_output_silu_mul(void *out, int out_dtype, 
         __half gh = __float2half_rn(g), uh = __float2half_rn(u);
         if (has_bias) { gh = __hadd(gh, bias_g); uh = __hadd(uh, bias_u); }
         __half c = __hmul(__float2half_rn(silu_f32(__half2float(gh))), uh);
-        if (ep.residual) c = __hadd(c, ep.residual[idx]);
+        if (ep.residual) c = __hadd(c, __ldcg(ep.residual + idx));
         reinterpret_cast<__half *>(out)[idx] = c;
     } else {
         if (has_bias) { g += __half2float(bias_g); u += __half2float(bias_u); }
         float v = silu_f32(g) * u;
-        if (ep.residual) v += __half2float(ep.residual[idx]);
+        if (ep.residual) v += __half2float(__ldcg(ep.residual + idx));
         if (out_dtype == BW_BF16) reinterpret_cast<__nv_bfloat16 *>(out)[idx] = __float2bfloat16_rn(v);
         else reinterpret_cast<float *>(out)[idx] = v;
     }

@@ -116,7 +116,7 @@ template <> __device__ __forceinline__ __half x_to_half<float>(float v) { return
 // 16-byte load:  xp[((chunk*NX + piece)*mt + m/8)*32 + (m%8)*4 + t].
 template <int BITS, typename XT>
 __global__ void __launch_bounds__(256)
-qmm_xprep_kernel(const XT *__restrict__ x, int64_t M, int64_t K, int mt, int chunks_total,
+qmm_xprep_kernel(const XT *x, int64_t M, int64_t K, int mt, int chunks_total,
                  uint4 *__restrict__ xp) {
     using Geo = Geometry<BITS>;
     constexpr int UNIT = Geo::UNIT;
@@ -135,7 +135,7 @@ qmm_xprep_kernel(const XT *__restrict__ x, int64_t M, int64_t K, int mt, int chu
         alignas(16) XT tmp[UNIT];
         const uint4 *src = reinterpret_cast<const uint4 *>(x + m * K + k);
 #pragma unroll
-        for (int j = 0; j < (int)(UNIT * sizeof(XT) / 16); ++j) reinterpret_cast<uint4 *>(tmp)[j] = __ldg(src + j);
+        for (int j = 0; j < (int)(UNIT * sizeof(XT) / 16); ++j) reinterpret_cast<uint4 *>(tmp)[j] = __ldcg(src + j);   // (from L2: see bw_common.cuh)
 #pragma unroll
         for (int e = 0; e < UNIT / 2; ++e)
             r[e] = h2_as_u32(__halves2half2(x_to_half<XT>(tmp[2 * e]), x_to_half<XT>(tmp[2 * e + 1])));

@@ -537,7 +537,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
 
 // Activations that are not fp16 are cast once (bitween/modules.py:74) into caller scratch.
 template <typename XT>
-__global__ void __launch_bounds__(256) cast_to_f16_kernel(const XT *__restrict__ x, __half *__restrict__ y, int64_t n, bool vec) {
+__global__ void __launch_bounds__(256) cast_to_f16_kernel(const XT *x, __half *y, int64_t n, bool vec) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");     // the GEMM behind it may start its set-up
     asm volatile("griddepcontrol.wait;" ::: "memory");                  // the kernel before may still write x or read y
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
@@ -546,16 +546,16 @@ __global__ void __launch_bounds__(256) cast_to_f16_kernel(const XT *__restrict__
         alignas(16) XT v[8];
         if (vec) {
 #pragma unroll
-            for (int j = 0; j < (int)sizeof(XT) / 2; ++j) reinterpret_cast<uint4 *>(v)[j] = reinterpret_cast<const uint4 *>(x + i)[j];
+            for (int j = 0; j < (int)sizeof(XT) / 2; ++j) reinterpret_cast<uint4 *>(v)[j] = __ldcg(reinterpret_cast<const uint4 *>(x + i) + j);   // (from L2: see bw_common.cuh)
         } else {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = x[i + j];
+            for (int j = 0; j < 8; ++j) v[j] = __ldcg(x + i + j);
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) h[j] = from_f32<__half>(to_f32<XT>(v[j]));
         *reinterpret_cast<uint4 *>(y + i) = *reinterpret_cast<const uint4 *>(h);
     } else {
-        for (int64_t j = i; j < n; ++j) y[j] = from_f32<__half>(to_f32<XT>(x[j]));
+        for (int64_t j = i; j < n; ++j) y[j] = from_f32<__half>(to_f32<XT>(__ldcg(x + j)));
     }
 }
 
