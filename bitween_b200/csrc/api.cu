@@ -98,6 +98,11 @@ static std::mutex &scratch_lock(const void *workspace) {
     return locks[(reinterpret_cast<uintptr_t>(workspace) >> 9) % 64];
 }
 
+static bool overlap(const void *a, size_t a_bytes, const void *b, size_t b_bytes) {
+    const uintptr_t p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
+    return p < q + b_bytes && q < p + a_bytes;
+}
+
 static bool is_float_dtype(int dt) { return dt == BW_F32 || dt == BW_F16 || dt == BW_BF16; }
 
 }  // namespace bw
@@ -245,7 +250,9 @@ static int qmatmul_dispatch(const void *x, int x_dtype, int64_t M, int64_t N, in
     //     otherwise 1 token 19200 x 2048 12.0 / 8.6, 28672 x 4096 22.7 / 18.5, 32768 x 8192 41.7 / 36.4, 3 tokens 41.8 / 37.1.
     const bool wide = decode && decode_shares_blocks(N), many = N * K >= (int64_t)1 << 25;
     const bool ring = (M > 6 && many) || (wide && (bits == 2 || M > 4 || N * K < (int64_t)1 << 24));
-    if (persistent_decode && rows_path_ok(x, x_dtype, M, N, K, qweight, bits, group_size) && !(decode && ring)) {
+    // (in place, the layouts of the cluster kernel stay on it: its preparation has read all of x before anything is stored)
+    const bool in_place = !decode && M <= 8 && overlap(x, (size_t)(M * K) * dtype_size(x_dtype), out, (size_t)(M * N) * dtype_size(out_dtype));
+    if (persistent_decode && !in_place && rows_path_ok(x, x_dtype, M, N, K, qweight, bits, group_size) && !(decode && ring)) {
         // (scratch is asked for wherever the kernel that would take over needs it)
         if ((!decode || wide) && (!workspace || !aligned_to(workspace, 16))) return BW_ERR_WORKSPACE;
         if (!decode && workspace_bytes < smallm_workspace_bytes(M, K, bits)) return BW_ERR_WORKSPACE;

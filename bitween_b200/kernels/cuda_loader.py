@@ -27,6 +27,7 @@ def quantized_matmul_cuda(x, qweight, scale, zero_point, bias, bits, group_size,
     optional fp16 bias [N].  Returns fp16 [..., N] exactly as the reference forward does
     (bitween/modules.py:106); `out_dtype` (bf16 / fp32) is an extension of this library.
 
+    `out`, a contiguous [M, N] tensor of out_dtype, takes the result; it may overlap `x` (which is copied then).
     `activation="relu"` and `residual` (fp16 [..., N], added last) fuse what follows the linear in
     a decoder block into the kernel's output stage (C ABI: bw_qmatmul_fused): the result equals
     `torch.relu(linear) + residual` computed op by op in fp16.  `activation="silu_mul"` is the
@@ -84,6 +85,9 @@ def quantized_matmul_cuda(x, qweight, scale, zero_point, bias, bits, group_size,
     else:
         if out.dtype != out_dtype or tuple(out.shape) != (M, N_out) or not out.is_contiguous() or out.device != dev:
             raise ValueError("`out` must be a contiguous [M, N] tensor of out_dtype on x's device ([M, N/2] for 'silu_mul')")
+        # some kernels store outputs while others of their CTAs still read x
+        if x2.data_ptr() < out.data_ptr() + out.nbytes and out.data_ptr() < x2.data_ptr() + x2.nbytes:
+            x2 = x2.clone()
     ep = None
     if activation is not None or residual is not None:
         if residual is not None:
@@ -204,7 +208,7 @@ def quantized_matmul_noalloc(x, qweight, scale, zero_point, bias, bits, group_si
     caller passes the output tensor, every tensor must already be a contiguous CUDA tensor of
     its final dtype (fp16 scale / zero_point / bias), and the kernel's scratch is a fixed 2 MiB
     array inside the library (C ABI: bw_qmatmul_noalloc).  Requests that need more scratch raise
-    BitweenKernelError (status 11).  All calls on one device share that array: issue them on
+    BitweenKernelError (status 11).  `out` must not overlap `x`.  All calls on one device share that array: issue them on
     one stream.  Make the first call on a device outside stream capture."""
     for name, t in (("x", x), ("qweight", qweight), ("scale", scale), ("zero_point", zero_point), ("out", out)):
         _lib.require_cuda(t, name)

@@ -137,7 +137,9 @@ BW_API int bw_dequantize(const int32_t *qweight, const void *scale, int scale_dt
  *   bias     [N] fp16 or NULL
  *   out      [M,N]  BW_F16: fp16(fp16(acc) + bias), the reference's two roundings
  *                   (bitween/modules.py:97,101); BW_BF16: bf16(acc + bias);
- *                   BW_F32: acc + bias with no 16-bit rounding (fp32-accumulate checks)
+ *                   BW_F32: acc + bias with no 16-bit rounding (fp32-accumulate checks).
+ *                   Must not overlap x, except where x is prepared or cast in the scratch first:
+ *                   layouts of the cluster kernel up to 64 tokens, and casts for the GEMM
  *   workspace       device scratch of at least bw_qmatmul_workspace_bytes(...) bytes, or
  *                   NULL when that is 0.  Calls that overlap on the GPU must not share it;
  *                   threads that call on one stream may (a call's launches stay together there);
