@@ -303,7 +303,12 @@ def run_decode8b(args, torch, dist, rank, world, device):
     clocks = sampler.stop()
     ms = max_over_ranks(torch, dist, device, ms)
     value = bytes_per_step * args.steps * world / (ms * 1e-3) / 1e9
-    decode_kernel = _lib.last_qmatmul_kernel()
+    ran = []                                               # the kernels of the sweep, in the order of its token counts
+    for M in DECODE_M:
+        for L in layers[0]:
+            quantized_matmul_cuda(xs[M][L.K], L.q, L.scale, L.zp, None, bits, g, out=outs[M][L.N])
+            ran.append(_lib.last_kernel())
+    decode_kernel = "+".join(dict.fromkeys(ran))
 
     # ---- end to end: pinned host activations in, host outputs back, per launch ----------
     hx = {M: {K: torch.randn(M, K).to(torch.bfloat16).pin_memory() for K in (4096, 14336)} for M in DECODE_M}
@@ -636,7 +641,7 @@ def run_tp70b(args, torch, dist, rank, world, device):
         "us_per_layer_without_allreduce": round(ms_no_ar * 1e3 / layers_n, 1),
         "allreduce_share": round(max(0.0, 1.0 - ms_no_ar / dec[best]), 3), "mode": best,
         "us_per_layer_by_mode": {k: round(v * 1e3 / layers_n, 1) for k, v in dec.items()},
-        "kernel": _lib.last_qmatmul_kernel(), "allreduce_bytes": 64 * HIDDEN70 * 2}
+        "kernel": _lib.last_kernel(), "allreduce_bytes": 64 * HIDDEN70 * 2}
     # the same decode step with the launches a decoder really issues: q/k/v as one column-parallel GEMM,
     # gate and up as one GEMM with the SiLU * up epilogue (interleaved row pairs), fp16 activations
     # throughout (no per-call cast): 4 GEMMs and 2 all-reduces per layer instead of 7 and 2

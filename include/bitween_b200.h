@@ -389,10 +389,11 @@ BW_API int bw_version(void);
  * and frees an 8-byte counter.
  */
 BW_API long long bw_selftest_division(unsigned long long n, unsigned long long seed);
-/* Name of the kernel the last bw_qmatmul call of this thread dispatched to (diagnostics).  Calls of at most 32
- * tokens go by the layout: "qmm_decode_kernel" (rows of scales and zero points in whole 16-byte units, and from 9 tokens on
- * those that are faster there) or "qmm_smallm_kernel" (others); most of both run on qmm_rows_kernel (up to 8 tokens) or
- * qmm_panel_kernel, which bw_last_kernel then names. */
+/* Which route the last bw_qmatmul call of this thread took, by its layout (diagnostics): "qmm_tc_kernel",
+ * "qmm_general_kernel", and up to 32 tokens "qmm_decode_kernel" (rows of scales and zero points in whole 16-byte units, and
+ * from 9 tokens on others that the ring kernel would take without scratch) or "qmm_smallm_kernel".  Up to 32 tokens this
+ * is a family of layouts, not the kernel that ran: most of both run on qmm_rows_kernel (up to 8 tokens) or
+ * qmm_panel_kernel.  bw_last_kernel names the kernel. */
 BW_API const char *bw_last_qmatmul_kernel(void);
 /* Name of the kernel that the last call of any kind on this thread ran (quantization, dequantization
  * and the backward pass included): which of several forms a layout took. */
