@@ -8,7 +8,9 @@ import contextlib
 import ctypes
 import importlib.util
 import os
+import sys
 import threading
+import warnings
 
 import torch
 
@@ -143,25 +145,36 @@ def lib():
     return _lib
 
 
+def _takes_no_call(*args):
+    return None
+
+
 _host = None
-HOST_LIB_PATH = os.path.join(_PKG, "_C", "_host_forward.so")
+# (compiled against torch's C++ interfaces: one for each Python and torch)
+HOST_LIB_PATH = os.path.join(_PKG, "_C", f"_host_forward.{sys.implementation.cache_tag}.torch-{torch.__version__}.so")
 
 
 def host_forward():
-    """The native host side of a layer's forward (csrc/host_forward.cpp), loaded with the library and built with it."""
+    """The native host side of a layer's forward (csrc/host_forward.cpp), loaded with the library and built with it.
+    Where it can be neither loaded nor built (no g++, no torch headers), that is reported once, and what is returned
+    takes no call: each goes through the autograd function, to the same kernels."""
     global _host
     if _host is None:
         L = lib()
         with _lock:
             if _host is None:
-                if not os.path.exists(HOST_LIB_PATH):
-                    from ..csrc.build import build
-                    build()
-                spec = importlib.util.spec_from_file_location("_host_forward", HOST_LIB_PATH)
-                module = importlib.util.module_from_spec(spec)
-                spec.loader.exec_module(module)
-                module.set_entry(ctypes.cast(L.bw_qmatmul, ctypes.c_void_p).value, _workspaces)
-                _host = module.forward
+                try:
+                    if not os.path.exists(HOST_LIB_PATH):
+                        from ..csrc.build import build_host
+                        build_host()
+                    spec = importlib.util.spec_from_file_location("_host_forward", HOST_LIB_PATH)
+                    module = importlib.util.module_from_spec(spec)
+                    spec.loader.exec_module(module)
+                    module.set_entry(ctypes.cast(L.bw_qmatmul, ctypes.c_void_p).value, _workspaces)
+                    _host = module.forward
+                except Exception as e:  # noqa: BLE001
+                    warnings.warn(f"bitween_b200: forwards run without the native host side ({e})", stacklevel=2)
+                    _host = _takes_no_call
     return _host
 
 
