@@ -24,6 +24,8 @@ def _layers(n, N, K, bits, g, gen):
     (12, 2048, 128, torch.float16, "qmm_panel_kernel"), (30, 1408, 128, torch.float32, "qmm_panel_kernel"),
     (5, 512, 16, torch.bfloat16, "qmm_smallm_kernel"),
     (48, 2048, 128, torch.float16, "qmm_tc_kernel"), (48, 2048, 128, torch.bfloat16, "qmm_tc_kernel"), (200, 1024, 128, torch.float32, "qmm_tc_kernel"),
+    # casts before 45 clusters of 3 and 26 of 5
+    (100, 5760, 128, torch.bfloat16, "qmm_tc_kernel"), (100, 3328, 128, torch.float32, "qmm_tc_kernel"),
 ])
 @pytest.mark.parametrize("residual", [False, True])
 def test_two_buffers_in_turn(tokens, K, g, dt, kernel, residual):
