@@ -246,13 +246,28 @@ static int qmatmul_dispatch(const void *x, int x_dtype, int64_t M, int64_t N, in
     // At most 8 tokens: the row kernel, but for some layers of the decode kernel's layout (us there / here, W4 g128):
     //   * from 7 tokens on, 2^25 weights or more: 8 tokens of bf16, 14336 x 4096, 13.6 / 14.4;
     //   * more row blocks than SMs (their shares travel through scratch there) with 2 bits (28672 x 1024, 1 token 9.4 / 10.4),
-    //     5 tokens or more (6 tokens, 28672 x 4096, 23.2 / 23.8; 24576 x 6144, W8, 34.9 / 53.6) or less than 2^24 weights;
+    //     5 tokens or more (6 tokens, 28672 x 4096, 23.2 / 23.8; 24576 x 6144, W8, 34.9 / 53.6) or less than 2^24 weights
+    //     (28709 x 512, 1 token, 8.4 / 11.1; 60 layers of 18945..32000 rows 541 / 599);
     //     otherwise 1 token 19200 x 2048 12.0 / 8.6, 28672 x 4096 22.7 / 18.5, 32768 x 8192 41.7 / 36.4, 3 tokens 41.8 / 37.1.
     const bool wide = decode && decode_shares_blocks(N), many = N * K >= (int64_t)1 << 25;
     const bool ring = (M > 6 && many) || (wide && (bits == 2 || M > 4 || N * K < (int64_t)1 << 24));
+    // Nor, in either layout (us of the ring or cluster kernel / here):
+    //   * short rows in more row tiles than CTAs (296), which follow one another while most warps of a CTA have no chunk (64 bytes
+    //     of a row) or one: 5530 x 320, W2, 3.5 / 4.8; 33405 x 448, W2, 6.0 / 17.1; 17111 x 384, W8, 6.8 / 8.9; 28442 x 704, W4, 9.3
+    //     / 14.1; 1152 columns are even.  190 of 489 random layers of 4737..34000 rows and 256..3072 columns, 1159 / 1715; the
+    //     others 3156 / 2714.
+    //   * with 16 warps a tile (launch_rows_warps) at 2 and 4 bits, longer rows too: 8 tokens, 21417 x 2944, W2, 15.7 / 28.2; 41
+    //     layers 892 / 1112.  The ring kernel's layouts of this kind are above.
+    //   * few rows with 128 KB of activations, which each CTA prepares for itself: 7 tokens of fp32, 275 x 10624, W4, 7.4 / 10.5;
+    //     18 layers 140 / 154.  (Up to 256 rows stay: the tests of long rows ask for this kernel there.)
+    const int64_t tiles = (N + 15) / 16, chunks = (K * bits + 511) / 512;
+    const bool flat = (tiles > 296 && chunks <= 3) || (tiles > 3 * 296 && (chunks <= 4 || K <= 512)) ||
+                      (tiles > 4 * 296 && (chunks <= 6 || K < 1024)) ||
+                      (!decode && M * K > 16384 && ((bits == 2 && N > 12000 && K < 4608) || (bits == 4 && N > 148 * 128 && K < 3072)));
+    const bool few = N > 256 && N <= 1280 && M * K * (int64_t)dtype_size(x_dtype) >= 128 << 10;
     // (in place, the layouts of the cluster kernel stay on it: its preparation has read all of x before anything is stored)
     const bool in_place = !decode && M <= 8 && overlap(x, (size_t)(M * K) * dtype_size(x_dtype), out, (size_t)(M * N) * dtype_size(out_dtype));
-    if (persistent_decode && !in_place && rows_path_ok(x, x_dtype, M, N, K, qweight, bits, group_size) && !(decode && ring)) {
+    if (persistent_decode && !in_place && rows_path_ok(x, x_dtype, M, N, K, qweight, bits, group_size) && !(decode && ring) && !flat && !few) {
         // (scratch is asked for wherever the kernel that would take over needs it)
         if ((!decode || wide) && (!workspace || !aligned_to(workspace, 16))) return BW_ERR_WORKSPACE;
         if (!decode && workspace_bytes < smallm_workspace_bytes(M, K, bits)) return BW_ERR_WORKSPACE;
