@@ -281,12 +281,18 @@ static int qmatmul_dispatch(const void *x, int x_dtype, int64_t M, int64_t N, in
     }
     std::unique_lock<std::mutex> together;
     if (workspace) together = std::unique_lock<std::mutex>(scratch_lock(workspace));
-    // 9 to 32 tokens: the panel kernel, but for layers of the decode kernel's layout that have more row blocks than SMs (16
-    // tokens, 24576 x 6144, W4: 34.0 us there, 39.1 here), 2^26 weights of 2 bits (19 layers of 9..16 tokens: 587 / 612), or,
-    // above 16 tokens, more than 9472 rows (51 such layers of 4096..8192 columns: 1828 / 1982); without scratch for the
-    // prepared activations the decode kernel takes what it can
-    if (persistent_decode && panel_path_ok(M, bits, group_size) &&
-        !(decode && (wide || (bits == 2 && N * K >= (int64_t)1 << 26) || (M > 16 && N > 4 * 148 * 16)))) {
+    // 9 to 32 tokens: the panel kernel, but for (us of the ring or cluster kernel / here; without scratch for the prepared
+    // activations the ring kernel takes what it can)
+    //   * layers of the ring kernel's layout that have more row blocks than SMs: 16 tokens, 24576 x 6144, W4, 34.0 / 39.1;
+    //   * its 2-bit layers of 2^26 weights: 19 of 9..16 tokens 587 / 612;
+    //   * above 16 tokens its 4-bit layers of long rows in 56 row blocks or more, whose pairs of CTAs then fill the SMs (17 tokens,
+    //     8532 x 10624, 38.9 / 48.3; 13 layers 529 / 603), and with groups of 32 those of 38 or more (11 layers 263 / 293);
+    //   * above 16 tokens all layers of more than 9472 rows: 51 of 4096..8192 columns on the ring kernel 1828 / 1982; 19 of
+    //     256..3776 columns on the cluster kernel 347 / 560 (17 tokens, 28691 x 384, 7.2 / 23.5);
+    //   * the cluster kernel's of more than 20000 very short rows: 12 tokens, 24477 x 256, W2, 4.6 / 9.0.
+    const bool long_rows = M > 16 && bits == 4 && ((N > 56 * 128 && K >= 6144) || (N > 2 * 148 * 16 && group_size == 32 && K >= 3400 && K < 8192));
+    if (persistent_decode && panel_path_ok(M, bits, group_size) && !(M > 16 && N > 4 * 148 * 16) && !(!decode && N > 20000 && K <= 384) &&
+        !(decode && (wide || (bits == 2 && N * K >= (int64_t)1 << 26) || long_rows))) {
         if (workspace && aligned_to(workspace, 16) && workspace_bytes >= smallm_workspace_bytes(M, K, bits)) {
             rc = qmatmul_panel(x, x_dtype, M, N, K, qweight, s, z, b, out, out_dtype, bits, group_size, workspace, st);
             if (rc == BW_OK) {

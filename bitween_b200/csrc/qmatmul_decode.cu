@@ -954,7 +954,8 @@ static bool dec_const_tma(const void *scale, const void *zp, int64_t K, int g) {
 //     x 9024, W4, 92 CTAs, 29 tokens: 42.7 / 33.8), with small groups (1536 x 8608, W4 g32, 30 tokens: 21.3 / 14.3) and in
 //     long rows, which it cuts into 8 pieces at most (768 x 21760, W4, 20 tokens: 34.4 / 21.8).
 // In sum over all 2718 calls 0.83 of the other kernel's time (0.87 if all were taken, 0.82 for the better one each
-// time); 102 lose more than 8 % (711 if all were taken).
+// time); 102 lose more than 8 % (711 if all were taken).  (Calls with scratch reach these lines above 16 tokens only, for more than
+// 9472 rows and the long rows that the dispatch names; the panel kernel has the others.)
 static bool dec_direct_consts(int64_t M, int64_t N, int64_t K, int bits, int g) {
     if (M <= 8 || N * K < (int64_t)1 << 22) return false;
     constexpr int64_t SMS = 148;

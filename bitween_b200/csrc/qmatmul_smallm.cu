@@ -748,7 +748,8 @@ int launch_panel(PanelParams p, cudaStream_t st) {
 //   14.6 / 13.5, W4 g32 22.0 / 17.7, W8 g128 18.8 / 18.0, W2 g64 18.2 / 13.3 (registers; 128 of them spill at 2 bits, one CTA
 //   of 64 rows an SM is slower still); 14208 x 1024, W4 g32 6.0 / 6.5;
 //   17..32 tokens: up to 2368 4101 / 2659 / 2818 / 3456 / 5053, to 4736 2762 / 2428 / 2819 / 2167 / 3433,
-//   to 9472 3229 / 2930 / 3469 / 3281 / 2925 (K from 8192 on 943 / 759 / 994 / 1026 / 963).
+//   to 9472 3229 / 2930 / 3469 / 3281 / 2925 (K from 8192 on 943 / 759 / 994 / 1026 / 963); above, the dispatch leaves them to the
+//   ring and cluster kernels.
 template <int BITS, int MT>
 int launch_panel_rows(const PanelParams &p, cudaStream_t st) {
     constexpr int OCC = MT <= 2 ? 2 : 1;
@@ -760,7 +761,7 @@ int launch_panel_rows(const PanelParams &p, cudaStream_t st) {
         if (p.N <= 6 * FULL && (BITS == 2 || p.K >= 1536)) return launch_panel<BITS, MT, 2, 3, 4, 2, 1>(p, st);
         return launch_panel<BITS, MT, 2, 2, 4, 2, OCC>(p, st);
     }
-    if (p.N <= 2 * FULL || p.N > 4 * FULL) return launch_panel<BITS, MT, 2, 1, 8, 2, OCC>(p, st);
+    if (p.N <= 2 * FULL) return launch_panel<BITS, MT, 2, 1, 8, 2, OCC>(p, st);
     if (p.K >= 8192) return launch_panel<BITS, MT, 1, 1, 16, 2, 1>(p, st);
     return launch_panel<BITS, MT, 2, 2, 4, 2, OCC>(p, st);
 }

@@ -38,10 +38,13 @@ def _without_scratch(x, q, s, z, b, bits, g, out):
     ("none", "qmm_decode_kernel", 4, 128, 13400, 1152, (16, 17)),
     # cluster kernel: groups of half a lane's codes
     ("scratch", "qmm_smallm_kernel", 4, 16, 1000, 1312, (1, 8, 9, 16, 17, 32)), ("scratch", "qmm_smallm_kernel", 8, 8, 130, 4112, (1, 8, 12, 32)),
-    # short rows of many row blocks, to either kernel; few rows of many activations
+    # short rows of many row blocks, to either kernel; few rows of many activations; above 16 tokens more than 9472 rows, long
+    # rows of 56 row blocks
     ("scratch", "qmm_smallm_kernel", 2, 64, 5530, 320, (1, 8)), ("scratch", "qmm_smallm_kernel", 4, 64, 19500, 704, (1, 3)),
     ("scratch", "qmm_smallm_kernel", 8, 32, 14300, 480, (2, 5)), ("scratch", "qmm_decode_kernel", 4, 32, 12222, 256, (1, 8)),
     ("scratch", "qmm_smallm_kernel", 2, 64, 12100, 2432, (7, 8)), ("scratch", "qmm_smallm_kernel", 4, 128, 937, 9600, (7, 8)),
+    ("scratch", "qmm_decode_kernel", 4, 128, 9473, 1408, (17, 32)), ("scratch", "qmm_smallm_kernel", 4, 128, 19100, 1408, (17, 32)), ("scratch", "qmm_smallm_kernel", 2, 128, 20100, 384, (9, 16, 24)),
+    ("scratch", "qmm_decode_kernel", 4, 128, 7200, 6144, (17, 32)), ("scratch", "qmm_decode_kernel", 4, 32, 4800, 3584, (24,)),
     # and with the scratch that is part of the library
     ("noalloc", "qmm_smallm_kernel", 2, 32, 1100, 2112, (1, 8, 9, 32)), ("noalloc", "qmm_smallm_kernel", 4, 128, 4737, 1408, (3, 16, 24)),
     ("noalloc", "qmm_smallm_kernel", 8, 64, 60, 9280, (2, 13, 30)),
