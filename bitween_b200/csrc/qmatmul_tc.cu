@@ -210,6 +210,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     asm volatile("griddepcontrol.wait;" ::: "memory");     // nothing has been read from or written to global memory before
+    if (p.ep.residual) __threadfence();
 
     if (warp == 0) {
         // ---- TMA producer of the activation tiles (one thread) ----
@@ -395,7 +396,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
             const int nblk = bn < 32 ? 1 : bn / 32, per = (nblk + TC_DQ_GROUPS - 1) / TC_DQ_GROUPS;
             const __half bias_h = (p.bias && n_ok) ? p.bias[n] : __float2half(0.0f);
             auto store_out = [&](int64_t m, float v) {
-                store_output(p.out, p.out_dtype, m * p.N + n, v, p.bias != nullptr, bias_h, p.ep);
+                store_output<true>(p.out, p.out_dtype, m * p.N + n, v, p.bias != nullptr, bias_h, p.ep);
             };
             if (p.splits == 1) {
                 if (TMAST && acc_ok) {
@@ -464,7 +465,7 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
                                 const float up = __shfl_xor_sync(0xffffffffu, __uint_as_float(r[j]), 1);
                                 const int64_t m = (int64_t)m0 + cb * 32 + j;
                                 if ((lane & 1) == 0 && n + 1 < p.N && n_ok && m < p.M)
-                                    store_output_silu_mul(p.out, p.out_dtype, m * (p.N >> 1) + (n >> 1), __uint_as_float(r[j]), up,
+                                    store_output_silu_mul<true>(p.out, p.out_dtype, m * (p.N >> 1) + (n >> 1), __uint_as_float(r[j]), up,
                                                           p.bias != nullptr, bias_h, bias_u, p.ep);
                             }
                             continue;
@@ -519,11 +520,11 @@ qmm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__
                     const float up = __shfl_xor_sync(0xffffffffu, v, 1);
                     const __half bias_u = __shfl_xor_sync(0xffffffffu, bias_h, 1);
                     if ((lane & 1) == 0 && n + 1 < p.N && m < p.M)
-                        store_output_silu_mul(p.out, p.out_dtype, m * (p.N >> 1) + (n >> 1), v, up, p.bias != nullptr, bias_h, bias_u, p.ep);
+                        store_output_silu_mul<true>(p.out, p.out_dtype, m * (p.N >> 1) + (n >> 1), v, up, p.bias != nullptr, bias_h, bias_u, p.ep);
                     continue;
                 }
                 if (n < p.N && m < p.M)
-                    store_output(p.out, p.out_dtype, m * p.N + n, v, p.bias != nullptr, bias_h, p.ep);
+                    store_output<true>(p.out, p.out_dtype, m * p.N + n, v, p.bias != nullptr, bias_h, p.ep);
             }
         }
         cluster.sync();   // keep shared memory alive until every peer has read it
