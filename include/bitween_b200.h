@@ -150,19 +150,23 @@ BW_API int bw_dequantize(const int32_t *qweight, const void *scale, int scale_dt
  *                   device), a captured graph owns its own until it is destroyed (beyond 448
  *                   live graphs the cluster kernel runs).  Make the first call on a device
  *                   outside a stream capture (it looks up the address of the counters).
- * Accumulation is fp32.  The kernel is chosen from M and the layout: up to 32 tokens run on
- * the persistent TMA-fed decode kernel (one launch; needs 16-byte aligned rows and K/group_size
- * to be a multiple of 8, or, from 9 tokens on, a layer whose grid makes loading the scales
- * directly pay; else the cluster split-K streaming kernel runs), more on the
- * tcgen05 tensor-core GEMM; unusual group sizes run on a slower general kernel, never on the
- * CPU.  The kernels are launched with programmatic dependent launch and fetch packed weights,
- * scales and zero points BEFORE waiting for the preceding kernel of the stream (only the
- * activations are read after it): qweight, scale and zero_point must not be written by the one
- * or two kernels that precede the call on its stream -- put an event or any non-library kernel
+ * Accumulation is fp32.  The kernel is chosen from M, N, K and the layout.  Most calls of up to 8
+ * tokens run on the row kernel (one launch, which uses no scratch) and of 9 to 32 on the panel
+ * kernel (a launch that prepares the activations in the scratch and one that reads them); layers
+ * that are faster there, and the gated output stage, on the persistent TMA-fed ring kernel (one
+ * launch; 16-byte aligned rows and K/group_size a multiple of 8) or, two launches again, on the
+ * cluster split-K kernel, which also takes groups smaller than a lane's 16 bytes of codes.  More
+ * tokens run on the tcgen05 tensor-core GEMM, behind a cast of activations that are not aligned
+ * fp16; unusual group sizes on a slower general kernel, never on the CPU.  Scratch is asked for by
+ * the layout, also where the row kernel then runs.  The kernels are launched with programmatic
+ * dependent launch, and those for up to 32 tokens fetch packed weights, scales and zero points
+ * BEFORE waiting for the preceding kernel of the stream (only the activations are read after it;
+ * the GEMM reads everything after it): qweight, scale and zero_point must not be written by the
+ * one or two kernels that precede the call on its stream -- put an event or any non-library kernel
  * between a weight update and the call.
- * bw_qmatmul_workspace_bytes: the prepared activations of the cluster kernel (K rounded
+ * bw_qmatmul_workspace_bytes: the prepared activations of the panel and cluster kernels (K rounded
  * up to a k-chunk x 8*ceil(min(M,64)/8) x 2 bytes), the fp16 cast of the activations for the
- * GEMM (M*K*2), or the decode kernel's row-block shares (320 x 8*ceil(M/8) x 128 x 4 bytes),
+ * GEMM (M*K*2), or the ring kernel's row-block shares (320 x 8*ceil(M/8) x 128 x 4 bytes),
  * whichever the call may need most.
  */
 BW_API size_t bw_qmatmul_workspace_bytes(int64_t M, int64_t N, int64_t K, int bits, int group_size);
